@@ -184,17 +184,20 @@ template <class E, int L, int IA, int IB, bool CTA = false>
 __device__ __forceinline__ void rc_exchange(E (&x)[RcLane<E>::P], E *buf,
                                             int g) {
   constexpr int P = RcLane<E>::P;
-  const int ba = rc_base<E, L, IA>(g), bb = rc_base<E, L, IB>(g);
+  // a lane's base and its registers' offsets occupy disjoint bits of the
+  // position (every factor is a power of two), so the padded address is the
+  // padded base plus a compile-time constant: no address arithmetic per
+  // access
+  E *const wa = buf + rc_pad<E, L>(rc_base<E, L, IA>(g));
+  const E *const ra = buf + rc_pad<E, L>(rc_base<E, L, IB>(g));
 #pragma unroll
-  for (int j = 0; j < P; ++j)
-    buf[rc_pad<E, L>(ba + rc_off<E, L, IA>(j))] = x[j];
+  for (int j = 0; j < P; ++j) wa[rc_pad<E, L>(rc_off<E, L, IA>(j))] = x[j];
   if constexpr (CTA)
     __syncthreads();
   else
     __syncwarp();
 #pragma unroll
-  for (int j = 0; j < P; ++j)
-    x[j] = buf[rc_pad<E, L>(bb + rc_off<E, L, IB>(j))];
+  for (int j = 0; j < P; ++j) x[j] = ra[rc_pad<E, L>(rc_off<E, L, IB>(j))];
   if constexpr (CTA)
     __syncthreads();
   else

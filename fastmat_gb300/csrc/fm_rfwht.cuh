@@ -133,16 +133,20 @@ __device__ __forceinline__ void rf_exchange(E (&x)[RfLane<E>::P], E *buf,
   constexpr int G = L / P;
   constexpr int WA = K - SA < PB ? K - SA : PB;
   constexpr int WB = K - SB < PB ? K - SB : PB;
+  // t, G u and r occupy disjoint bits of the position, so the padded address
+  // is the thread's padded base plus a compile-time constant
+  E *const wa = buf + rf_xpad<E>(rf_pos(t, SA, 0, WA));
+  const E *const ra = buf + rf_xpad<E>(rf_pos(t, SB, 0, WB));
 #pragma unroll
   for (int j = 0; j < P; ++j) {
     const int u = j >> WA, r = j & ((1 << WA) - 1);
-    buf[rf_xpad<E>(rf_pos(t + G * u, SA, r, WA))] = x[j];
+    wa[rf_xpad<E>(rf_pos(G * u, SA, r, WA))] = x[j];
   }
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < P; ++j) {
     const int u = j >> WB, r = j & ((1 << WB) - 1);
-    x[j] = buf[rf_xpad<E>(rf_pos(t + G * u, SB, r, WB))];
+    x[j] = ra[rf_xpad<E>(rf_pos(G * u, SB, r, WB))];
   }
   __syncthreads();
 }
@@ -204,11 +208,12 @@ __device__ __forceinline__ void rf_finish(
   if (act) {
     const unsigned m = dA.div((unsigned)gv);
     const unsigned a = (unsigned)gv - m * (unsigned)p.A;
-    Raw *dst = (Raw *)p.dst + (i64)m * p.ld_dst + (i64)a * p.stride;
+    Raw *dst = (Raw *)p.dst + (i64)m * p.ld_dst + (i64)a * p.stride +
+               rf_pos(t, SL, 0, WL);
 #pragma unroll
     for (int j = 0; j < P; ++j) {
       const int u = j >> WL, r = j & ((1 << WL) - 1);
-      const int e = rf_pos(t + G * u, SL, r, WL);
+      const int e = rf_pos(G * u, SL, r, WL);
       if constexpr (Emu<E>::v)
         dst[e] = df2d_scaled(x[j], s);
       else
@@ -324,8 +329,11 @@ __device__ __forceinline__ void rs_batch(const RfStep &p, i64 bt, E *xb,
   const i64 row0 = (i64)a * L * S + c0 + v;
   const Raw *src = (const Raw *)p.src + (i64)m * p.ld_src + row0;
   Raw d[P];
+  {
+    const Raw *q = src + (i64)(t * P) * S;
 #pragma unroll
-  for (int r = 0; r < P; ++r) d[r] = src[(i64)(t * P + r) * S];
+    for (int r = 0; r < P; ++r, q += S) d[r] = *q;
+  }
   E x[P];
   int s = 0;
   if constexpr (Emu<E>::v) {
@@ -349,15 +357,18 @@ __device__ __forceinline__ void rs_batch(const RfStep &p, i64 bt, E *xb,
   // separate this batch's reads of sexp from the next batch's reset)
   static_assert(W >= 2, "threads per vector");
   rf_passes<E, L, 0>(x, buf, t);
-  Raw *dst = (Raw *)p.dst + (i64)m * p.ld_dst + row0;
+  Raw *dst = (Raw *)p.dst + (i64)m * p.ld_dst + row0 +
+             (i64)rf_pos(t, SL, 0, WL) * S;
 #pragma unroll
-  for (int j = 0; j < P; ++j) {
-    const int u = j >> WL, r = j & ((1 << WL) - 1);
-    const int e = rf_pos(t + W * u, SL, r, WL);
-    if constexpr (Emu<E>::v)
-      dst[(i64)e * S] = df2d_scaled(x[j], s);
-    else
-      dst[(i64)e * S] = x[j];
+  for (int u = 0; u < (P >> WL); ++u) {
+    Raw *q = dst + (i64)rf_pos(W * u, SL, 0, WL) * S;
+#pragma unroll
+    for (int r = 0; r < (1 << WL); ++r, q += S << SL) {
+      if constexpr (Emu<E>::v)
+        *q = df2d_scaled(x[(u << WL) + r], s);
+      else
+        *q = x[(u << WL) + r];
+    }
   }
 }
 

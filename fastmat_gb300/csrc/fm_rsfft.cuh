@@ -86,8 +86,11 @@ __global__ void __launch_bounds__(RsfShape<E, L>::T, (RsfOcc<E>::v))
     const i64 row0 = (i64)a * L * Sx + c0 + v;
     const Raw *src = (const Raw *)p.src + (i64)m * p.ld_src + row0;
     Raw d[P];
+    {
+      const Raw *q = src + (i64)t * Sx;
 #pragma unroll
-    for (int r = 0; r < P; ++r) d[r] = src[(i64)(t + G * r) * Sx];
+      for (int r = 0; r < P; ++r, q += G * Sx) d[r] = *q;
+    }
     E x[P];
     int s = 0;
     if constexpr (Emu<E>::v) {
@@ -110,16 +113,22 @@ __global__ void __launch_bounds__(RsfShape<E, L>::T, (RsfOcc<E>::v))
     // (S >= 2: the stages hold at least one exchange, whose barriers also
     // separate this batch's reads of sexp from the next batch's reset)
     rc_forward<E, L, 0, SG, true>(x, buf, t, stw);
-    Raw *dst = (Raw *)p.dst + (i64)m * p.ld_dst + row0;
-    const int bl = rc_base<E, L, S - 1>(t);
+    // register u R + r of the last stage (radix R) holds the natural index
+    // of the thread's base plus u R + r L / R
+    constexpr int R = rc_radix(S - 1, L, P);
+    Raw *dst = (Raw *)p.dst + (i64)m * p.ld_dst + row0 +
+               (i64)rc_nat<E, L>(rc_base<E, L, S - 1>(t)) * Sx;
 #pragma unroll
-    for (int j = 0; j < P; ++j) {
-      const int nat = rc_nat<E, L>(bl + rc_off<E, L, S - 1>(j));
-      if constexpr (Emu<E>::v)
-        dst[(i64)nat * Sx] = make_double2(df2d_scaled(x[j].x, s),
-                                          df2d_scaled(x[j].y, s));
-      else
-        dst[(i64)nat * Sx] = x[j];
+    for (int u = 0; u < P / R; ++u) {
+      Raw *q = dst + (i64)(u * R) * Sx;
+#pragma unroll
+      for (int r = 0; r < R; ++r, q += (L / R) * Sx) {
+        const E y = x[u * R + r];
+        if constexpr (Emu<E>::v)
+          *q = make_double2(df2d_scaled(y.x, s), df2d_scaled(y.y, s));
+        else
+          *q = y;
+      }
     }
   }
 }
