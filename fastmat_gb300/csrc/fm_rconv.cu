@@ -56,7 +56,7 @@ int rconv_max_len(int ctype) {
 }
 int rconv_min_len(int ctype) {
   return ctype == FM_C64 ? RcLane<float2>::P
-         : ctype == FM_C128_DF ? RcLane<dfc>::P
+         : ctype == FM_C128_DF ? RcLane<dfq>::P
                                : 0;
 }
 int rconv_lane_points(int ctype) { return rconv_min_len(ctype); }
@@ -74,12 +74,12 @@ cudaError_t launch_rconv(int ctype, const RcStep &p, cudaStream_t s) {
     }
   } else if (ctype == FM_C128_DF) {
     switch (p.L) {
-      case 8: return launch_one<dfc, 8>(p, s);
-      case 16: return launch_one<dfc, 16>(p, s);
-      case 32: return launch_one<dfc, 32>(p, s);
-      case 64: return launch_one<dfc, 64>(p, s);
-      case 128: return launch_one<dfc, 128>(p, s);
-      case 256: return launch_one<dfc, 256>(p, s);
+      case 8: return launch_one<dfq, 8>(p, s);
+      case 16: return launch_one<dfq, 16>(p, s);
+      case 32: return launch_one<dfq, 32>(p, s);
+      case 64: return launch_one<dfq, 64>(p, s);
+      case 128: return launch_one<dfq, 128>(p, s);
+      case 256: return launch_one<dfq, 256>(p, s);
       default: break;
     }
   }

@@ -72,7 +72,8 @@ __global__ void __launch_bounds__(FM_RCH_THREADS, (RchOcc<E>::v))
   constexpr int S1 = Sh::S1;
   constexpr int NV2 = Sh::NV2;
   static_assert(G >= 1 && G <= 32 && NV2 >= 1, "layout");
-  typedef typename std::conditional<Emu<E>::v, double2, E>::type Raw;
+  typedef E Raw;
+  static_assert(!Emu<E>::v, "single precision");
   extern __shared__ __align__(128) unsigned char fm_smem[];
   unsigned *sitem = reinterpret_cast<unsigned *>(fm_smem);
   E *stw = reinterpret_cast<E *>(fm_smem + 16);
@@ -80,7 +81,7 @@ __global__ void __launch_bounds__(FM_RCH_THREADS, (RchOcc<E>::v))
   unsigned char *region =
       fm_smem + 16 + ((size_t)(Sh::TWN + L1) * sizeof(E) + 15) / 16 * 16;
   const int tid = threadIdx.x;
-  rc_fill_tw<E, L1, 0>(stw, (const E *)p.c.tw);
+  rc_fill_tw<E, L1, 0>(stw, p.c.tw);
   // the spectrum in lane-major order (as the register convolution keeps it)
   for (int i = tid; i < L1; i += FM_RCH_THREADS) {
     const int j = i / G, gg = i % G;
@@ -140,23 +141,8 @@ __global__ void __launch_bounds__(FM_RCH_THREADS, (RchOcc<E>::v))
 #pragma unroll
       for (int r = 0; r < P; ++r) d[r] = src[g + G * r];
       E x[P];
-      int s = 0;
-      if constexpr (Emu<E>::v) {
-        int emax = 0;
 #pragma unroll
-        for (int r = 0; r < P; ++r)
-          emax = max(emax, max(dexp(d[r].x), dexp(d[r].y)));
-#pragma unroll
-        for (int o = G / 2; o >= 1; o /= 2)
-          emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o, G));
-        s = emax > 0 ? emax - 1023 : 0;
-#pragma unroll
-        for (int r = 0; r < P; ++r)
-          x[r] = dfc{d2df_scaled(d[r].x, s), d2df_scaled(d[r].y, s)};
-      } else {
-#pragma unroll
-        for (int r = 0; r < P; ++r) x[r] = d[r];
-      }
+      for (int r = 0; r < P; ++r) x[r] = d[r];
       rc_forward<E, L1, 0>(x, buf, g, stw);
 #pragma unroll
       for (int j = 0; j < P; ++j)
@@ -165,13 +151,7 @@ __global__ void __launch_bounds__(FM_RCH_THREADS, (RchOcc<E>::v))
       Raw *dst = (Raw *)p.c.dst + (i64)m * p.c.ld_dst +
                  (i64)a * p.c.out_stride;
 #pragma unroll
-      for (int r = 0; r < P; ++r) {
-        if constexpr (Emu<E>::v)
-          dst[g + G * r] = make_double2(df2d_scaled(x[r].x, s),
-                                        df2d_scaled(x[r].y, s));
-        else
-          dst[g + G * r] = x[r];
-      }
+      for (int r = 0; r < P; ++r) dst[g + G * r] = x[r];
       // this item's stores, then its count (release)
       __syncthreads();
       if (tid == 0) {

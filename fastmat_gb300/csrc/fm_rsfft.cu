@@ -73,11 +73,11 @@ cudaError_t launch_rsfft(int ctype, const RsfStep &p, cudaStream_t s) {
     }
   } else if (ctype == FM_C128_DF) {
     switch (p.L) {
-      case 16: return launch_signed<dfc, 16>(p, s);
-      case 32: return launch_signed<dfc, 32>(p, s);
-      case 64: return launch_signed<dfc, 64>(p, s);
-      case 128: return launch_signed<dfc, 128>(p, s);
-      case 256: return launch_signed<dfc, 256>(p, s);
+      case 16: return launch_signed<dfq, 16>(p, s);
+      case 32: return launch_signed<dfq, 32>(p, s);
+      case 64: return launch_signed<dfq, 64>(p, s);
+      case 128: return launch_signed<dfq, 128>(p, s);
+      case 256: return launch_signed<dfq, 256>(p, s);
       default: break;
     }
   }

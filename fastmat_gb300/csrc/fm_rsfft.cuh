@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(RsfShape<E, L>::T, (RsfOcc<E>::v))
   E *stw = reinterpret_cast<E *>(fm_smem);
   E *xb = stw + TWN;
   int *sexp = reinterpret_cast<int *>(xb + NV * Sh::Lx);
-  rc_fill_tw<E, L, 0>(stw, (const E *)p.tw);
+  rc_fill_tw<E, L, 0>(stw, p.tw);
   __syncthreads();
   const int v = threadIdx.x % NV, t = threadIdx.x / NV;
   E *buf = xb + v * Sh::Lx;
@@ -94,18 +94,13 @@ __global__ void __launch_bounds__(RsfShape<E, L>::T, (RsfOcc<E>::v))
     E x[P];
     int s = 0;
     if constexpr (Emu<E>::v) {
-      int emax = 0;
-#pragma unroll
-      for (int r = 0; r < P; ++r)
-        emax = max(emax, max(dexp(d[r].x), dexp(d[r].y)));
+      const int emax = rx_max<P>(d);
       if (threadIdx.x < NV) sexp[threadIdx.x] = 0;
       __syncthreads();
       if (emax > 0) atomicMax(sexp + v, emax);
       __syncthreads();
-      s = sexp[v] > 0 ? sexp[v] - 1023 : 0;
-#pragma unroll
-      for (int r = 0; r < P; ++r)
-        x[r] = dfc{d2df_scaled(d[r].x, s), d2df_scaled(d[r].y, s)};
+      s = df_scale(sexp[v] >> 20);
+      rx_in<P>(x, d, s);
     } else {
 #pragma unroll
       for (int r = 0; r < P; ++r) x[r] = d[r];
@@ -118,18 +113,9 @@ __global__ void __launch_bounds__(RsfShape<E, L>::T, (RsfOcc<E>::v))
     constexpr int R = rc_radix(S - 1, L, P);
     Raw *dst = (Raw *)p.dst + (i64)m * p.ld_dst + row0 +
                (i64)rc_nat<E, L>(rc_base<E, L, S - 1>(t)) * Sx;
-#pragma unroll
-    for (int u = 0; u < P / R; ++u) {
-      Raw *q = dst + (i64)(u * R) * Sx;
-#pragma unroll
-      for (int r = 0; r < R; ++r, q += (L / R) * Sx) {
-        const E y = x[u * R + r];
-        if constexpr (Emu<E>::v)
-          *q = make_double2(df2d_scaled(y.x, s), df2d_scaled(y.y, s));
-        else
-          *q = y;
-      }
-    }
+    rx_out<P>(x, s, [&](int j, Raw y) {
+      dst[((i64)((j / R) * R) + (j % R) * (L / R)) * Sx] = y;
+    });
   }
 }
 

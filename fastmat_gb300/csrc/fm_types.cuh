@@ -120,6 +120,90 @@ __device__ __forceinline__ dfcu operator-(dfcu a, dfcu b) {
   return dfcu{a.x - b.x, a.y - b.y};
 }
 
+// ---- complex double-float in packed form: the heads of real and imaginary
+// part as one float2, the tails as another, so that every operation on both
+// parts is one packed FP32 instruction (add / sub / mul / fma .rn.f32x2:
+// each half rounds exactly as the scalar operation).  The packed forms run
+// at the scalar FP32 rate but take half the issue slots (measured: 64
+// packed or 128 scalar additions per clock and SM), which the register
+// kernels' conversion and exchange instructions then use.  dfq is
+// normalised as dfc is, dfqu unnormalised as dfcu is.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n .reg .b64 a, b, c;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n"
+      " add.rn.f32x2 c, a, b;\n mov.b64 {%0, %1}, c;\n}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n .reg .b64 a, b, c;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n"
+      " sub.rn.f32x2 c, a, b;\n mov.b64 {%0, %1}, c;\n}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n .reg .b64 a, b, c;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n"
+      " mul.rn.f32x2 c, a, b;\n mov.b64 {%0, %1}, c;\n}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 d) {
+  float2 r;
+  asm("{\n .reg .b64 a, b, c, d;\n mov.b64 a, {%2, %3};\n"
+      " mov.b64 b, {%4, %5};\n mov.b64 d, {%6, %7};\n"
+      " fma.rn.f32x2 c, a, b, d;\n mov.b64 {%0, %1}, c;\n}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(d.x), "f"(d.y));
+  return r;
+}
+__device__ __forceinline__ float2 neg2(float2 a) {
+  return make_float2(-a.x, -a.y);
+}
+struct dfq {
+  float2 h, l;  // (re, im) heads, (re, im) tails
+};
+struct dfqu {
+  float2 h, l;
+};
+__device__ __forceinline__ dfq pack(dfc a) {
+  return dfq{make_float2(a.x.h, a.y.h), make_float2(a.x.l, a.y.l)};
+}
+__device__ __forceinline__ dfc unpack(dfq a) {
+  return dfc{df(a.h.x, a.l.x), df(a.h.y, a.l.y)};
+}
+__device__ __forceinline__ dfqu operator+(dfqu a, dfqu b) {
+  const float2 s = add2(a.h, b.h);
+  const float2 bb = sub2(s, a.h);
+  const float2 e = add2(sub2(a.h, sub2(s, bb)), sub2(b.h, bb));
+  return dfqu{s, add2(add2(a.l, b.l), e)};
+}
+__device__ __forceinline__ dfqu operator-(dfqu a, dfqu b) {
+  const float2 s = sub2(a.h, b.h);
+  const float2 bb = sub2(s, a.h);
+  const float2 e = sub2(sub2(a.h, sub2(s, bb)), add2(b.h, bb));
+  return dfqu{s, add2(sub2(a.l, b.l), e)};
+}
+// product with a real factor (h, l) common to both parts
+__device__ __forceinline__ dfqu rmul(dfqu a, float h, float l) {
+  const float2 bh = make_float2(h, h), bl = make_float2(l, l);
+  const float2 p = mul2(a.h, bh);
+  float2 e = fma2(a.h, bh, neg2(p));
+  e = fma2(a.h, bl, e);
+  e = fma2(a.l, bh, e);
+  return dfqu{p, e};
+}
+// a times i (sign > 0) or -i
+__device__ __forceinline__ dfqu rot90(dfqu a, int sign) {
+  if (sign > 0)
+    return dfqu{make_float2(-a.h.y, a.h.x), make_float2(-a.l.y, a.l.x)};
+  return dfqu{make_float2(a.h.y, -a.h.x), make_float2(a.l.y, -a.l.x)};
+}
+
 // double -> double-float with integer operations only (the FP64 pipe of
 // this GPU is slow): h is d rounded to 24 bits, l the float nearest to the
 // exact remainder d - h.  Zeros, subnormals and values outside the float
@@ -211,10 +295,21 @@ template <> struct Tr<dfcu> {
   static constexpr int code = FM_C128;
   typedef dfu R;
 };
+template <> struct Tr<dfq> {
+  static constexpr bool cplx = true;
+  static constexpr int code = FM_C128;
+  typedef df R;
+};
+template <> struct Tr<dfqu> {
+  static constexpr bool cplx = true;
+  static constexpr int code = FM_C128;
+  typedef dfu R;
+};
 // the type a butterfly computes in: unnormalised for double-float
 template <class C> struct Lazy { typedef C type; };
 template <> struct Lazy<df> { typedef dfu type; };
 template <> struct Lazy<dfc> { typedef dfcu type; };
+template <> struct Lazy<dfq> { typedef dfqu type; };
 template <class C> __device__ __forceinline__ C to_lazy(C a) { return a; }
 template <class C> __device__ __forceinline__ C from_lazy(C a) { return a; }
 __device__ __forceinline__ dfu to_lazy(df a) { return dfu(a.h, a.l); }
@@ -227,7 +322,13 @@ __device__ __forceinline__ df from_lazy(dfu a) {
 __device__ __forceinline__ dfc from_lazy(dfcu a) {
   return dfc{fast_two_sum(a.x.h, a.x.l), fast_two_sum(a.y.h, a.y.l)};
 }
+__device__ __forceinline__ dfqu to_lazy(dfq a) { return dfqu{a.h, a.l}; }
+__device__ __forceinline__ dfq from_lazy(dfqu a) {
+  const float2 s = add2(a.h, a.l);
+  return dfq{s, sub2(a.l, sub2(s, a.h))};
+}
 template <class E> struct Emu { static constexpr bool v = false; };
+template <> struct Emu<dfq> { static constexpr bool v = true; };
 template <> struct Emu<df> { static constexpr bool v = true; };
 template <> struct Emu<dfc> { static constexpr bool v = true; };
 
@@ -288,6 +389,17 @@ __device__ __forceinline__ df mulv(df a, df b, bool) { return a * b; }
 __device__ __forceinline__ dfc mulv(dfc a, dfc b, bool c) {
   return c ? cmulc(a, b) : cmul(a, b);
 }
+// (packed form: the unnormalised product, renormalised once)
+__device__ __forceinline__ dfq mulv(dfq a, dfq b, bool c) {
+  const float2 by = c ? make_float2(-b.h.y, -b.l.y)
+                      : make_float2(b.h.y, b.l.y);
+  const dfqu u = to_lazy(a);
+  return from_lazy(rmul(u, b.h.x, b.l.x) +
+                   rmul(rot90(u, +1), by.x, by.y));
+}
+__device__ __forceinline__ dfq conjv(dfq a) {
+  return dfq{make_float2(a.h.x, -a.h.y), make_float2(a.l.x, -a.l.y)};
+}
 __device__ __forceinline__ df conjv(df a) { return a; }
 __device__ __forceinline__ dfc conjv(dfc a) { return dfc{a.x, -a.y}; }
 __device__ __forceinline__ df addv(df a, df b) { return a + b; }
@@ -347,6 +459,9 @@ template <> __device__ __forceinline__ df scalar_of<df>(double re, double) {
 }
 template <> __device__ __forceinline__ dfc scalar_of<dfc>(double re, double im) {
   return dfc{d2df(re), d2df(im)};
+}
+template <> __device__ __forceinline__ dfq scalar_of<dfq>(double re, double im) {
+  return pack(dfc{d2df(re), d2df(im)});
 }
 
 __device__ __forceinline__ float addv(float a, float b) { return a + b; }
@@ -651,6 +766,81 @@ __device__ __forceinline__ void store_as(void *p, int type, i64 idx, E v,
     }
     default: return;
   }
+}
+
+// element i of a plan's table (twiddles, spectra, products; dfc in memory
+// for the packed form)
+template <class E>
+__device__ __forceinline__ E tab_get(const void *p, i64 i) {
+  if constexpr (sizeof(E) == 16 && Emu<E>::v && Tr<E>::cplx)
+    return pack(((const dfc *)p)[i]);
+  else
+    return ((const E *)p)[i];
+}
+template <class E>
+__device__ __forceinline__ void store_elem(void *p, int type, i64 idx, E v,
+                                           bool acc, int scale = 0) {
+  if constexpr (Emu<E>::v)
+    store_as<dfc>(p, type, idx, unpack(v), acc, scale);
+  else
+    store_as<E>(p, type, idx, v, acc, scale);
+}
+
+// ---- float64 <-> packed double-float in the register kernels.  A vector
+// is scaled by 2^-s, s = its largest exponent minus kDfTop, so its largest
+// element sits at 2^kDfTop; elements more than 2^(74 + kDfTop) below it
+// (2^-114, far below the 2^-48 of the arithmetic) flush to zero.
+// A vector holding Inf or NaN gets the s that maps the exponent field of
+// Inf / NaN to float's, so those elements stay Inf / NaN.
+constexpr int kDfTop = 40;
+// largest (hi & 0x7fffffff) of a vector's words -> s
+__device__ __forceinline__ int df_scale(int emax) {
+  return emax >= 0x7FF ? 896 : emax - 1023 - kDfTop;
+}
+// s for which no result can leave the float64 range (results lie within
+// 2^-127 .. 2^127 of 2^s)
+__device__ __forceinline__ bool df_scale_plain(int s) {
+  return s >= -890 && s <= 890;
+}
+// d 2^-s as h + l: h the leading 24 significand bits (truncated), l the
+// other 29 rounded to a float.  sub = (s + 896) << 23, thr = the smallest
+// high word (sign cleared) that does not flush.
+__device__ __forceinline__ void d2hl(double d, unsigned sub, int thr,
+                                     float &h, float &l) {
+  const unsigned hi = (unsigned)__double2hiint(d),
+                 lo = (unsigned)__double2loint(d);
+  const unsigned sg = hi & 0x80000000u;
+  // exponent field (9 bits) and 23 significand bits, exponent rebased
+  const unsigned t = __funnelshift_l(lo, hi, 3) - sub;
+  // the remaining bits weigh 2^(ef - 127 - 52) each
+  const float f = __int_as_float((int)((t & 0x7F800000u) - (52u << 23)));
+  const float r = (float)(lo & 0x1FFFFFFFu) * f;
+  const bool keep = (int)(hi & 0x7FFFFFFFu) >= thr;
+  h = keep ? __int_as_float((int)(t | sg)) : 0.f;
+  l = keep ? __int_as_float((int)(__float_as_int(r) | sg)) : 0.f;
+}
+// (h + l) 2^s as a float64, rounded to nearest: h's bits widened exactly, l
+// converted to units in the last place of that float64 and added to its bit
+// pattern (an integer addition: carries move into the exponent as they
+// should).  bias = (s + 896) << 20; s plain (df_scale_plain).
+__device__ __forceinline__ double hl2d(float h, float l, int bias) {
+  const unsigned u = (unsigned)__float_as_int(h);
+  const unsigned eb = u & 0x7F800000u;
+  // +-2^(52 - e): one unit of the result's last place is 2^(e - 52)
+  const float w =
+      __int_as_float((int)(((306u << 23) - eb) | (u & 0x80000000u)));
+  int n = __float2int_rn(l * w);
+  // below a power of two the spacing halves
+  if ((u & 0x007FFFFFu) == 0u && n < 0) n += n;
+  const unsigned hi = ((unsigned)((int)u >> 3) & 0x8FFFFFFFu) + (unsigned)bias;
+  const unsigned lo = u << 29;
+  i64 b = (i64)(((unsigned long long)hi << 32) | lo) + (i64)n;
+  if (eb == 0u) b = 0;
+  return __longlong_as_double(b);
+}
+// the largest exponent word of raw points
+__device__ __forceinline__ int raw_hi(double d) {
+  return __double2hiint(d) & 0x7FFFFFFF;
 }
 
 }  // namespace fmk

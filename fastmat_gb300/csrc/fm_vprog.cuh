@@ -298,6 +298,17 @@ __device__ __forceinline__ C twc(C x, int sign) {
     return x;
   } else if constexpr (idx == 4) {
     return rot90(x, sign);  // * (i sign)
+  } else if constexpr (std::is_same<C, dfqu>::value) {
+    // packed: x c + (i x) sn; at odd multiples of pi / 4 one product of
+    // the sum
+    constexpr dfu c = dfu(kCos16(idx)), sp = dfu(kSin16(idx));
+    const dfqu y = rot90(x, sign);
+    if constexpr (idx == 2)
+      return rmul(x + y, c.h, c.l);
+    else if constexpr (idx == 6)
+      return rmul(y - x, sp.h, sp.l);
+    else
+      return rmul(x, c.h, c.l) + rmul(y, sp.h, sp.l);
   } else {
     const R c = (R)kCos16(idx), sp = (R)kSin16(idx);
     const R sn = sign < 0 ? -sp : sp;
@@ -461,6 +472,11 @@ __device__ __forceinline__ LC cmul_lazy(LC a, C w) {
     return SG < 0 ? cmul(a, w) : cmulc(a, w);
   } else {
     const LC b = to_lazy(w);
+    if constexpr (std::is_same<LC, dfqu>::value) {
+      // a w = a Re w + (i a) Im w
+      return rmul(a, b.h.x, b.l.x) +
+             rmul(rot90(a, SG < 0 ? +1 : -1), b.h.y, b.l.y);
+    } else {
     LC r;
     if constexpr (SG < 0) {
       r.x = a.x * b.x - a.y * b.y;
@@ -470,6 +486,7 @@ __device__ __forceinline__ LC cmul_lazy(LC a, C w) {
       r.y = a.y * b.x - a.x * b.y;
     }
     return r;
+    }
   }
 }
 
