@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include "fm_rconv.cuh"
+#include "fm_rfft.cuh"
 #include "fm_rfwht.cuh"
 #include "fm_rsfft.cuh"
 #include "fm_rpair.cuh"
@@ -76,6 +77,16 @@ int rsfwht_max_len(int ctype);
 int rsfft_min_len(int ctype);
 int rsfft_max_len(int ctype);
 cudaError_t launch_rsfft(int ctype, const RsfStep &p, cudaStream_t s);
+// register transforms of long vectors (fm_rfft.cuh), complex64 and
+// double-float complex: FFTs of strided vectors (lengths rxfft_min ..
+// rxfft_max, contiguous input up to rxfft_max_turn) and convolutions of
+// contiguous vectors (rxconv_min .. rxconv_max), powers of two
+constexpr int rxfft_min = 32, rxfft_max = 512, rxfft_max_turn = 1024;
+constexpr int rxconv_min = 64, rxconv_max = 4096;
+cudaError_t launch_rxfft_c64(const RxStep &p, cudaStream_t s);
+cudaError_t launch_rxfft_df(const RxStep &p, cudaStream_t s);
+cudaError_t launch_rxconv_c64(const RxStep &p, cudaStream_t s);
+cudaError_t launch_rxconv_df(const RxStep &p, cudaStream_t s);
 // a circulant Kron mode and the Hadamard mode after it in one launch
 // (rkch_kernel): whether it is built for the lengths and a block's items
 // divide evenly (n1 / n2: convolution / FWHT items per block)

@@ -200,6 +200,58 @@ __global__ void k_twiddle2(E *tw, i64 N, int s) {
   }
 }
 
+// element in the register kernels' own type (packed double-float)
+template <class E> __device__ E mkx(double re, double im) {
+  return mk<E>(re, im);
+}
+template <> __device__ fmk::dfq mkx<fmk::dfq>(double re, double im) {
+  return fmk::pack(mk<fmk::dfc>(re, im));
+}
+
+// Stage twiddle tables of the register transforms of length L with P points
+// per thread (rc_twoff): for every stage with radix R, Mprev = the length
+// left and M = Mprev / R > 1, entry k M + t = exp(-2 pi i t k / Mprev).
+template <class E>
+__global__ void k_rx_twiddle(E *tw, int L, int P, int total) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total;
+       i += gridDim.x * blockDim.x) {
+    int e = i, mp = L;
+    while (e >= mp) {  // every stage before the last holds Mprev entries
+      e -= mp;
+      mp /= mp < P ? mp : P;
+    }
+    const int M = mp / (mp < P ? mp : P);
+    const int k = e / M, t = e - k * M;
+    double s, c;
+    sincospi(-2.0 * (double)(t * k) / (double)mp, &s, &c);
+    tw[i] = mkx<E>(c, s);
+  }
+}
+
+// Four-step twiddles w[j N2 + q] = exp(-2 pi i j q / N), j < N / N2.
+template <class E>
+__global__ void k_rx_wtab(E *w, i64 N, i64 N2) {
+  for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < N;
+       i += (i64)gridDim.x * blockDim.x) {
+    const i64 j = i / N2, q = i - j * N2;
+    double s, c;
+    sincospi(-2.0 * (double)((j * q) % N) / (double)N, &s, &c);
+    w[i] = mkx<E>(c, s);
+  }
+}
+
+// Spectra in the register convolution's order: out[v L + i] =
+// in[v stride + perm[i]], i < L, v < n (in: the plan's compute type)
+template <class E>
+__global__ void k_rx_spec(E *out, const void *in, const int *perm, i64 L,
+                          i64 n, i64 stride) {
+  for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < L * n;
+       i += (i64)gridDim.x * blockDim.x) {
+    const i64 v = i / L;
+    out[i] = fmk::tab_get<E>(in, v * stride + perm[i - v * L]);
+  }
+}
+
 // Bluestein chirp a[n] = exp(-i pi n^2 / N) with n^2 reduced mod 2N exactly
 __global__ void k_chirp(double2 *a, i64 N) {
   for (i64 n = blockIdx.x * (i64)blockDim.x + threadIdx.x; n < N;
@@ -249,7 +301,8 @@ struct LStep {
   // first row of the launch's operand inside its buffer (Blocks segments)
   i64 src_off = 0, dst_off = 0;
   // 0: vector program (vprog_kernel); 1: CSR sparse product (spmv_kernel);
-  // 2: register-resident convolution (rconv_kernel), 3: register-resident
+  // 2: register-resident convolution (rconv_kernel), 5 / 6: register FFT /
+  // convolution of long vectors (rxfft_kernel / rxconv_kernel), 3: register-resident
   // FWHT (rfwht_kernel / rsfwht_kernel / rfwht2_kernel), 4: register FFT of
   // strided vectors (rsfft_kernel); for 2..4 `st` still holds the
   // equivalent vector program (run by batches, and when the buffers do not
@@ -275,6 +328,10 @@ struct LStep {
   const void *rc_spec = nullptr, *rc_tw = nullptr;  // spectrum in rconv order
   const void *rc_pre = nullptr, *rc_post = nullptr;
   int rc_conj_in = 0, rc_conj_out = 0, rc_spec_conj = 0;
+  // kinds 5, 6: four-step twiddles, products by point, spectrum stride
+  const void *rx_w = nullptr;
+  i64 rx_wq = 0, rx_wj = 0, rx_spec_stride = 0;
+  int rx_w_sign = 0, rx_pre_pt = 0, rx_post_pt = 0;
   const i64 *sp_ptr = nullptr, *sp_idx = nullptr;
   const void *sp_val = nullptr;
   i64 sp_rows = 0;
@@ -1866,11 +1923,179 @@ class Planner {
     ls.kind = 4;
   }
 
+  // ---- tables of the register transforms of long vectors (fm_rfft.cuh)
+  std::map<i64, const void *> rx_tw_;
+  std::map<std::pair<i64, i64>, const void *> rx_w_;
+  const void *rx_twiddle(int L) {
+    auto it = rx_tw_.find(L);
+    if (it != rx_tw_.end()) return it->second;
+    const int P = fmk::kRxP;
+    int total = 0;  // stages with M > 1
+    for (int mp = L; mp > P; mp /= P) total += mp;
+    void *p = dalloc((size_t)total * P_->esz);
+    if (P_->ctype == FM_C64)
+      k_rx_twiddle<float2><<<grid_for(total), 256>>>((float2 *)p, L, P, total);
+    else
+      k_rx_twiddle<fmk::dfq><<<grid_for(total), 256>>>((fmk::dfq *)p, L, P,
+                                                       total);
+    CUDA_TRY(cudaGetLastError());
+    return rx_tw_[L] = p;
+  }
+  const void *rx_wtab(i64 N, i64 N2) {
+    const std::pair<i64, i64> key(N, N2);
+    auto it = rx_w_.find(key);
+    if (it != rx_w_.end()) return it->second;
+    void *p = dalloc((size_t)N * P_->esz);
+    if (P_->ctype == FM_C64)
+      k_rx_wtab<float2><<<grid_for(N), 256>>>((float2 *)p, N, N2);
+    else
+      k_rx_wtab<fmk::dfq><<<grid_for(N), 256>>>((fmk::dfq *)p, N, N2);
+    CUDA_TRY(cudaGetLastError());
+    return rx_w_[key] = p;
+  }
+  // spectra in the order the lanes hold the forward transform's results
+  const void *rx_spectrum(const void *in, int L, i64 n, i64 stride) {
+    const int P = fmk::kRxP, G = L / P;
+    std::vector<int> rad;
+    for (int rest = L; rest > 1; rest /= rad.back())
+      rad.push_back(std::min(rest, P));
+    const Perm &pm = perm_for(rad);
+    const int R = rad.back();  // last stage: M = 1
+    std::vector<int> perm((size_t)L);
+    for (int j = 0; j < P; ++j)
+      for (int g = 0; g < G; ++g)
+        perm[(size_t)(j * G + g)] =
+            pm.nat[(size_t)(g * R + (j / R) * G * R + j % R)];
+    DevTemp tp;
+    CUDA_TRY(dev_malloc(&tp.p, (size_t)L * sizeof(int)));
+    CUDA_TRY(cudaMemcpy(tp.p, perm.data(), (size_t)L * sizeof(int),
+                        cudaMemcpyHostToDevice));
+    void *p = dalloc((size_t)(L * n) * P_->esz);
+    if (P_->ctype == FM_C64)
+      k_rx_spec<float2><<<grid_for(L * n), 256>>>(
+          (float2 *)p, in, (const int *)tp.p, L, n, stride);
+    else
+      k_rx_spec<fmk::dfq><<<grid_for(L * n), 256>>>(
+          (fmk::dfq *)p, in, (const int *)tp.p, L, n, stride);
+    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(cudaDeviceSynchronize());
+    return p;
+  }
+
+  // A program that is one FFT over vectors whose results leave strided
+  // (kind 5: strided vectors, or contiguous ones stored transposed), or one
+  // circular convolution of contiguous vectors (kind 6), with the loader's
+  // and storer's work around it and an optional four-step twiddle at its
+  // end, runs in the register transforms of long vectors when its length is
+  // a power of two they are built for.  Lines of the rule: strided vectors
+  // need rows of at least 64 bytes (two sectors; narrower ones load no
+  // better there than in the stage kernel's tiles); a plain Fourier mode of
+  // a Kron above 512 points, and a whole Fourier column in one launch, stay
+  // on the stage kernel's tiles.
+  void try_rx(LStep &ls, const std::vector<fmk::Op> &ops) {
+    const int ct = P_->ctype;
+    if (ct != FM_C64 && ct != FM_C128_DF) return;
+    const fmk::Step &st = ls.st;
+    if (st.out_mode == 1 || st.has_scale) return;
+    auto whole = [](const fmk::Op &o) {
+      return o.kind == fmk::OP_MUL && o.div == 1 && o.mod == 1 &&
+             o.stride == 0 && o.sign == 0;
+    };
+    auto is = [&](size_t i, int kind) {
+      return i < ops.size() && ops[i].kind == kind;
+    };
+    size_t i = 0;
+    bool cj_in = false, cj_out = false;
+    const void *pre = nullptr, *post = nullptr;
+    if (is(i, fmk::OP_CONJ)) cj_in = true, ++i;
+    if (i < ops.size() && whole(ops[i]) && ops[i].len >= st.in_len &&
+        (is(i + 1, fmk::OP_ZPAD) || is(i + 1, fmk::OP_FFT)))
+      pre = ops[i++].ptr;
+    if (is(i, fmk::OP_ZPAD)) {
+      if (ops[i].len != st.in_len) return;
+      ++i;
+    }
+    if (!is(i, fmk::OP_FFT)) return;
+    const int L = ops[i].len, sign = ops[i].sign;
+    ++i;
+    const fmk::Op *sm = nullptr;
+    if (is(i, fmk::OP_MUL) && is(i + 1, fmk::OP_FFT)) {
+      sm = &ops[i];
+      if (sign != -1 || ops[i + 1].sign != 1 || ops[i + 1].len != L ||
+          sm->len != L || sm->div != 1 ||
+          !((sm->mod == 1 && sm->stride == 0) ||
+            (sm->mod == st.V && sm->stride >= L)))
+        return;
+      i += 2;
+    }
+    const fmk::Op *tw = nullptr;
+    if (is(i, fmk::OP_TW)) {
+      tw = &ops[i];
+      if (tw->len != L || tw->div != 1 || tw->mod != st.V ||
+          tw->N != (i64)L * st.V)
+        return;
+      ++i;
+    } else {
+      if (i < ops.size() && whole(ops[i]) && ops[i].len >= st.out_len)
+        post = ops[i++].ptr;
+      if (is(i, fmk::OP_CONJ)) cj_out = true, ++i;
+    }
+    if (i != ops.size()) return;
+    if (!is_pow2(L) || st.L != L || st.in_len > L || st.out_len > L ||
+        st.vin.A * st.vin.Cc != st.V || st.vout.A * st.vout.Cc != st.V)
+      return;
+    if ((pre && st.pre) || (post && st.post) || (cj_in && st.conj_in) ||
+        (cj_out && st.conj_out))
+      return;
+    const i64 ci = st.vin.Cc, co = st.vout.Cc;
+    const i64 wide = 64 / P_->esz;
+    if (sm) {
+      if (ci != 1 || co != 1 || L < fmk::rxconv_min || L > fmk::rxconv_max)
+        return;
+    } else {
+      if (co < wide || (ci != 1 && ci < wide) || L < fmk::rxfft_min ||
+          L > (ci == 1 ? fmk::rxfft_max_turn : fmk::rxfft_max))
+        return;
+    }
+    ls.rc_L = L;
+    ls.rc_tw = rx_twiddle(L);
+    ls.rc_pre = pre;
+    ls.rc_post = post;
+    ls.rx_pre_pt = pre != nullptr;
+    ls.rx_post_pt = post != nullptr;
+    ls.rc_conj_in = cj_in;
+    ls.rc_conj_out = cj_out;
+    ls.rc_sign = sign;
+    if (sm) {
+      const bool per = sm->mod != 1;
+      ls.rc_spec = rx_spectrum(sm->ptr, L, per ? st.V : 1, sm->stride);
+      ls.rx_spec_stride = per ? L : 0;
+      ls.rc_spec_conj = sm->sign;
+    }
+    if (tw) {
+      // one table per (N, N2), entry j N2 + q of row j < N1: the pass over
+      // vectors of N1 points has j the point and q the vector, the pass over
+      // vectors of N2 points the reverse
+      if (ci != 1) {
+        ls.rx_w = rx_wtab(tw->N, st.V);
+        ls.rx_wq = 1;
+        ls.rx_wj = st.V;
+      } else {
+        ls.rx_w = rx_wtab(tw->N, L);
+        ls.rx_wq = L;
+        ls.rx_wj = 1;
+      }
+      ls.rx_w_sign = tw->sign;
+    }
+    ls.kind = sm ? 6 : 5;
+  }
+
   void finish(LStep &ls, const std::vector<fmk::Op> &ops_in) {
     fmk::Step &st = ls.st;
     try_rconv(ls, ops_in);
     if (ls.kind == 0) try_rfwht(ls, ops_in);
     if (ls.kind == 0) try_rsfft(ls, ops_in);
+    if (ls.kind == 0) try_rx(ls, ops_in);
     std::vector<fmk::Op> ops = ops_in;
     st.out_pos = finalize(ops);
     if ((int)ops.size() > FM_MAX_OPS)
@@ -2386,6 +2611,60 @@ void launch_step(fm_plan *P, LStep &ls, fmk::Step &st, cudaStream_t s) {
       return;
     }
     // otherwise the equivalent vector program below
+  }
+  if (ls.kind == 5 || ls.kind == 6) {
+    fmk::RxStep rx;
+    memset(&rx, 0, sizeof(rx));
+    rx.src = st.src;
+    rx.dst = st.dst;
+    rx.ld_src = st.ld_src;
+    rx.ld_dst = st.ld_dst;
+    rx.src_type = st.src_type;
+    rx.dst_type = st.dst_type;
+    rx.V = st.V;
+    rx.in_n = st.vin.n;
+    rx.in_cc = st.vin.Cc;
+    rx.out_n = st.vout.n;
+    rx.out_cc = st.vout.Cc;
+    rx.in_rows = st.in_rows;
+    rx.out_rows = st.out_rows;
+    rx.num_cols = st.num_cols;
+    rx.map_in = st.map_in;
+    rx.map_out = st.out_mode == 2 ? st.map_out : nullptr;
+    rx.pre = st.pre ? st.pre : ls.rc_pre;
+    rx.post = st.post ? st.post : ls.rc_post;
+    rx.pre_by_point = ls.rx_pre_pt;
+    rx.post_by_point = ls.rx_post_pt;
+    rx.spec = ls.rc_spec;
+    rx.spec_stride = ls.rx_spec_stride;
+    rx.tw = ls.rc_tw;
+    rx.wtab = ls.rx_w;
+    rx.wq = ls.rx_wq;
+    rx.wj = ls.rx_wj;
+    rx.in_len = st.in_len;
+    rx.out_len = st.out_len;
+    // an inverse FFT is the conjugate of the forward FFT of the conjugate
+    const int inv = ls.kind == 5 && ls.rc_sign > 0;
+    rx.conj_in = (st.conj_in || ls.rc_conj_in) != inv;
+    rx.conj_out = (st.conj_out || ls.rc_conj_out) != inv;
+    rx.pre_conj = inv;
+    rx.post_conj = inv;
+    rx.w_conj = (ls.rx_w_sign > 0) != inv;
+    rx.spec_conj = ls.rc_spec_conj;
+    rx.has_scale = st.has_scale;
+    rx.scale_re = st.scale_re;
+    rx.scale_im = inv ? -st.scale_im : st.scale_im;
+    rx.accumulate = st.accumulate;
+    rx.L = ls.rc_L;
+    if (rx.V * rx.num_cols >= 0x7fffffffLL)
+      fail(FM_ERR_UNSUPPORTED, "more than 2^31 vectors in one launch");
+    const bool single = P->ctype == FM_C64;
+    CUDA_TRY(ls.kind == 5
+                 ? (single ? fmk::launch_rxfft_c64(rx, s)
+                           : fmk::launch_rxfft_df(rx, s))
+                 : (single ? fmk::launch_rxconv_c64(rx, s)
+                           : fmk::launch_rxconv_df(rx, s)));
+    return;
   }
   if (ls.kind == 2) {
     fmk::RcStep rc;
@@ -3252,16 +3531,27 @@ int fm_plan_describe(const fm_plan *plan, int32_t direction, char *buf,
         s += line;
         continue;
       }
-      if (ls.kind == 2) {
+      if (ls.kind == 2 || ls.kind == 5 || ls.kind == 6) {
         snprintf(line, sizeof(line),
                  "launch src=%d dst=%d in=(%lld,%lld,%lld) out=(%lld,%lld,"
-                 "%lld) rconv L=%d acc=%d:",
+                 "%lld) %s L=%d acc=%d:",
                  ls.src, ls.dst, st.vin.A, st.vin.n, st.vin.Cc, st.vout.A,
-                 st.vout.n, st.vout.Cc, ls.rc_L, st.accumulate);
+                 st.vout.n, st.vout.Cc,
+                 ls.kind == 2   ? "rconv"
+                 : ls.kind == 5 ? "rxfft"
+                                : "rxconv",
+                 ls.rc_L, st.accumulate);
         s += line;
         s += ls.rc_conj_in || st.conj_in ? " conj" : "";
         s += ls.rc_pre || st.pre ? " pre" : "";
-        s += " fft-conv";
+        if (ls.kind == 5) {
+          snprintf(line, sizeof(line), " fft(%d, sign %d)", ls.rc_L,
+                   ls.rc_sign);
+          s += line;
+        } else {
+          s += " fft-conv";
+        }
+        if (ls.rx_w) s += " twiddle";
         s += ls.rc_post || st.post ? " post" : "";
         s += ls.rc_conj_out || st.conj_out ? " conj" : "";
         s += ls.pair == 3 ? " fused-with-next" : "";

@@ -68,6 +68,9 @@ struct RcStep {
 template <class E> struct RcLane {
   static constexpr int P = sizeof(E) == 8 ? 16 : 8;
 };
+template <int NP> struct RcLane<cfp<NP>> {
+  static constexpr int P = NP;
+};
 
 // Shared-memory layout of a vector's exchange buffer: point p at
 // p + (p >> SH), vectors Lp points apart; its input slot: natural order,
@@ -76,8 +79,8 @@ template <class E> struct RcLane {
 // (the stage layouts' exchange writes and reads and the slot reads, per
 // half- or quarter-warp phase): all are conflict-free except the exchange
 // of L = 32 (4 wavefronts where 3 would do, on average); the twiddle and
-// spectrum tables are read lane-major (consecutive lanes, consecutive
-// entries) and broadcast across the vectors of a warp.
+// spectrum tables are read by consecutive lanes at consecutive entries and
+// broadcast across the vectors of a warp.
 template <class E, int L> struct RcBuf {
   static constexpr bool C64 = sizeof(E) == 8;
   static constexpr int SH =
@@ -90,12 +93,19 @@ template <class E, int L> struct RcBuf {
   static constexpr int Ls = C64 ? (L <= 128 ? L + L / 16 : L)
                                 : (L <= 32 ? L + L / 8 : L);
 };
+// (packed complex64 of the long-vector transforms, fm_rfft.cuh: same
+// enumeration, at most 1.5 wavefronts per access where 1 would do)
+template <int L> struct RcBuf<cfp<8>, L> {
+  static constexpr int SH = 3;
+  static constexpr int Lp = L + (L >> 3);
+};
 template <class E, int L> __device__ __forceinline__ int rc_pad(int p) {
   return p + (p >> RcBuf<E, L>::SH);
 }
 
-// Offset of stage I's lane-major twiddle table (R_I x G entries, stages
-// with M > 1 only) within the twiddle area of shared memory.
+// Offset of stage I's twiddle table (R_I x M_I entries w_Mprev^(t k) at
+// k M + t, stages with M > 1 only) within the launch's twiddle tables.
+// Consecutive lanes read consecutive (or the same) entries.
 template <class E, int L, int I>
 __host__ __device__ constexpr int rc_twoff() {
   constexpr int P = RcLane<E>::P;
@@ -104,7 +114,7 @@ __host__ __device__ constexpr int rc_twoff() {
   } else {
     constexpr int R = rc_radix(I - 1, L, P);
     constexpr int M = rc_mprev(I - 1, L, P) / R;
-    return rc_twoff<E, L, I - 1>() + (M > 1 ? R * (L / P) : 0);
+    return rc_twoff<E, L, I - 1>() + (M > 1 ? R * M : 0);
   }
 }
 template <class E, int L, int I>
@@ -116,7 +126,22 @@ __host__ __device__ constexpr int rc_twlen() {  // entries of stages < I
 // or inverse (INV = true: conjugate twiddles of the inputs, then DFT with
 // sign +1) transform on the lane's P registers, in place: register
 // u R + r holds position base + u G R + M r before and after.
-template <class E, int L, int I, bool INV, int FSG = -1>
+// element i of a stage's twiddle table: shared memory, or (GT) global
+// memory in the element type itself, read through the L1 cache
+template <bool GT, class E>
+__device__ __forceinline__ E tw_get(const E *tab, int i) {
+  if constexpr (!GT) {
+    return tab[i];
+  } else if constexpr (sizeof(E) == 16) {
+    const float4 v = __ldg(reinterpret_cast<const float4 *>(tab) + i);
+    return *reinterpret_cast<const E *>(&v);
+  } else {
+    const float2 v = __ldg(reinterpret_cast<const float2 *>(tab) + i);
+    return *reinterpret_cast<const E *>(&v);
+  }
+}
+
+template <class E, int L, int I, bool INV, int FSG = -1, bool GT = false>
 __device__ __forceinline__ void rc_stage(E (&x)[RcLane<E>::P], int g,
                                          const E *__restrict__ stw) {
   constexpr int P = RcLane<E>::P;
@@ -124,19 +149,15 @@ __device__ __forceinline__ void rc_stage(E (&x)[RcLane<E>::P], int g,
   constexpr int Mprev = rc_mprev(I, L, P);
   constexpr int M = Mprev / R;
   constexpr int NB = P / R;
-  constexpr int TS = L / Mprev;  // table stride of w_Mprev
   constexpr int SG = INV ? +1 : FSG;  // FSG: sign of a forward-order DIF
   typedef typename Lazy<E>::type LC;
-  constexpr int G = L / P;
-  // the twiddles w_Mprev^(t k), t = g mod M, k < R, are the same for all
-  // u: lane-major table of this stage (entry k G + g), conflict-free reads
+  // the twiddles w_Mprev^(t k), t = g mod M, k < R, are the same for all u
   E w[R];
   if constexpr (M > 1) {
-    const E *tab = stw + rc_twoff<E, L, I>();
+    const E *tab = stw + rc_twoff<E, L, I>() + (g & (M - 1));
 #pragma unroll
-    for (int k = 1; k < R; ++k) w[k] = tab[k * G + g];
+    for (int k = 1; k < R; ++k) w[k] = tw_get<GT>(tab, k * M);
   }
-  (void)TS;
 #pragma unroll
   for (int u = 0; u < NB; ++u) {
     LC v[R];
@@ -204,14 +225,15 @@ __device__ __forceinline__ void rc_exchange(E (&x)[RcLane<E>::P], E *buf,
     __syncwarp();
 }
 
-template <class E, int L, int I, int FSG = -1, bool CTA = false>
+template <class E, int L, int I, int FSG = -1, bool CTA = false,
+          bool GT = false>
 __device__ __forceinline__ void rc_forward(E (&x)[RcLane<E>::P], E *buf, int g,
                                            const E *stw) {
-  rc_stage<E, L, I, false, FSG>(x, g, stw);
+  rc_stage<E, L, I, false, FSG, GT>(x, g, stw);
   constexpr int S = rc_stages(L, RcLane<E>::P);
   if constexpr (I + 1 < S) {
     rc_exchange<E, L, I, I + 1, CTA>(x, buf, g);
-    rc_forward<E, L, I + 1, FSG, CTA>(x, buf, g, stw);
+    rc_forward<E, L, I + 1, FSG, CTA, GT>(x, buf, g, stw);
   }
 }
 
@@ -242,13 +264,13 @@ template <class E, int L>
 __device__ __forceinline__ int rc_nat(int p) {
   return rc_nat_from<E, L, 0>(p, 0);
 }
-template <class E, int L, int I>
+template <class E, int L, int I, bool CTA = false, bool GT = false>
 __device__ __forceinline__ void rc_inverse(E (&x)[RcLane<E>::P], E *buf, int g,
                                            const E *stw) {
-  rc_stage<E, L, I, true>(x, g, stw);
+  rc_stage<E, L, I, true, -1, GT>(x, g, stw);
   if constexpr (I > 0) {
-    rc_exchange<E, L, I, I - 1>(x, buf, g);
-    rc_inverse<E, L, I - 1>(x, buf, g, stw);
+    rc_exchange<E, L, I, I - 1, CTA>(x, buf, g);
+    rc_inverse<E, L, I - 1, CTA, GT>(x, buf, g, stw);
   }
 }
 
@@ -297,7 +319,7 @@ __device__ __forceinline__ void rx_out(const E (&x)[P], int s, F store) {
     }
   } else {
 #pragma unroll
-    for (int r = 0; r < P; ++r) store(r, x[r]);
+    for (int r = 0; r < P; ++r) store(r, make_float2(x[r].x, x[r].y));
   }
 }
 
@@ -317,9 +339,9 @@ __host__ __device__ constexpr size_t rc_smem() {
          sizeof(E);
 }
 
-// Fill the lane-major twiddle tables of stages I.. from the natural table
-// tw[j] = exp(-2 pi i j / L): entry k G + g of stage I is w_Mprev^(t k),
-// t = g mod M (the stage's table stride L / Mprev in tw).
+// Fill the twiddle tables of stages I.. from the natural table
+// tw[j] = exp(-2 pi i j / L): entry k M + t of stage I is w_Mprev^(t k)
+// (the stage's table stride L / Mprev in tw).
 template <class E, int L, int I>
 __device__ __forceinline__ void rc_fill_tw(E *stw, const void *tw) {
   constexpr int P = RcLane<E>::P;
@@ -328,12 +350,11 @@ __device__ __forceinline__ void rc_fill_tw(E *stw, const void *tw) {
     constexpr int R = rc_radix(I, L, P);
     constexpr int Mprev = rc_mprev(I, L, P);
     constexpr int M = Mprev / R;
-    constexpr int G = L / P;
     if constexpr (M > 1) {
       E *tab = stw + rc_twoff<E, L, I>();
-      for (int i = threadIdx.x; i < R * G; i += blockDim.x) {
-        const int k = i / G, g = i % G;
-        tab[i] = tab_get<E>(tw, (g & (M - 1)) * k * (L / Mprev));
+      for (int i = threadIdx.x; i < R * M; i += blockDim.x) {
+        const int k = i / M, t = i % M;
+        tab[i] = tab_get<E>(tw, t * k * (L / Mprev));
       }
     }
     rc_fill_tw<E, L, I + 1>(stw, tw);

@@ -1,0 +1,20 @@
+// Instantiations and launcher of rxconv_kernel (fm_rfft.cuh): complex64.
+#include "fm_launch.cuh"
+#include "fm_rfft.cuh"
+
+namespace fmk {
+
+cudaError_t launch_rxconv_c64(const RxStep &p, cudaStream_t s) {
+  switch (p.L) {
+    case 64: return rxconv_one<cfp<8>, 64>(p, s);
+    case 128: return rxconv_one<cfp<8>, 128>(p, s);
+    case 256: return rxconv_one<cfp<8>, 256>(p, s);
+    case 512: return rxconv_one<cfp<8>, 512>(p, s);
+    case 1024: return rxconv_one<cfp<8>, 1024>(p, s);
+    case 2048: return rxconv_one<cfp<8>, 2048>(p, s);
+    case 4096: return rxconv_one<cfp<8>, 4096>(p, s);
+    default: return cudaErrorInvalidConfiguration;
+  }
+}
+
+}  // namespace fmk

@@ -188,6 +188,36 @@ __device__ __forceinline__ dfqu operator-(dfqu a, dfqu b) {
   const float2 e = sub2(sub2(a.h, sub2(s, bb)), add2(b.h, bb));
   return dfqu{s, add2(sub2(a.l, b.l), e)};
 }
+// complex64 with packed additions, NP points per thread in the register
+// transforms (the results of every operation are float2's)
+template <int NP> struct alignas(8) cfp {
+  float x, y;
+};
+template <int NP>
+__device__ __forceinline__ cfp<NP> operator+(cfp<NP> a, cfp<NP> b) {
+  const float2 r = add2(make_float2(a.x, a.y), make_float2(b.x, b.y));
+  return cfp<NP>{r.x, r.y};
+}
+template <int NP>
+__device__ __forceinline__ cfp<NP> operator-(cfp<NP> a, cfp<NP> b) {
+  const float2 r = sub2(make_float2(a.x, a.y), make_float2(b.x, b.y));
+  return cfp<NP>{r.x, r.y};
+}
+template <int NP>
+__device__ __forceinline__ cfp<NP> cmul(cfp<NP> a, cfp<NP> b) {
+  return cfp<NP>{fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x)};
+}
+template <int NP>
+__device__ __forceinline__ cfp<NP> cmulc(cfp<NP> a, cfp<NP> b) {
+  return cfp<NP>{fmaf(a.x, b.x, a.y * b.y), fmaf(a.y, b.x, -a.x * b.y)};
+}
+template <int NP>
+__device__ __forceinline__ cfp<NP> mulv(cfp<NP> a, cfp<NP> b, bool c) {
+  return c ? cmulc(a, b) : cmul(a, b);
+}
+template <int NP> __device__ __forceinline__ cfp<NP> conjv(cfp<NP> a) {
+  return cfp<NP>{a.x, -a.y};
+}
 // product with a real factor (h, l) common to both parts
 __device__ __forceinline__ dfqu rmul(dfqu a, float h, float l) {
   const float2 bh = make_float2(h, h), bl = make_float2(l, l);
@@ -294,6 +324,11 @@ template <> struct Tr<dfcu> {
   static constexpr bool cplx = true;
   static constexpr int code = FM_C128;
   typedef dfu R;
+};
+template <int NP> struct Tr<cfp<NP>> {
+  static constexpr bool cplx = true;
+  static constexpr int code = FM_C64;
+  typedef float R;
 };
 template <> struct Tr<dfq> {
   static constexpr bool cplx = true;
@@ -438,7 +473,9 @@ template <> __device__ __forceinline__ dfc zero<dfc>() {
 
 // a (complex) scalar given in double precision, in the element type E;
 // for double-float types this is the host-free integer split
-template <class E> __device__ __forceinline__ E scalar_of(double re, double im);
+template <class E> __device__ __forceinline__ E scalar_of(double re, double im) {
+  return E{(float)re, (float)im};
+}
 template <> __device__ __forceinline__ float scalar_of<float>(double re, double) {
   return (float)re;
 }
@@ -783,16 +820,19 @@ __device__ __forceinline__ void store_elem(void *p, int type, i64 idx, E v,
   if constexpr (Emu<E>::v)
     store_as<dfc>(p, type, idx, unpack(v), acc, scale);
   else
-    store_as<E>(p, type, idx, v, acc, scale);
+    store_as<float2>(p, type, idx, make_float2(v.x, v.y), acc);
 }
 
 // ---- float64 <-> packed double-float in the register kernels.  A vector
 // is scaled by 2^-s, s = its largest exponent minus kDfTop, so its largest
 // element sits at 2^kDfTop; elements more than 2^(74 + kDfTop) below it
-// (2^-114, far below the 2^-48 of the arithmetic) flush to zero.
+// (2^-84, far below the 2^-48 of the arithmetic) flush to zero.  kDfTop
+// leaves the operator's own magnitude most of float's exponent range on
+// both sides (results 2^-109 .. 2^117 of the largest element keep their
+// tails).
 // A vector holding Inf or NaN gets the s that maps the exponent field of
 // Inf / NaN to float's, so those elements stay Inf / NaN.
-constexpr int kDfTop = 40;
+constexpr int kDfTop = 10;
 // largest (hi & 0x7fffffff) of a vector's words -> s
 __device__ __forceinline__ int df_scale(int emax) {
   return emax >= 0x7FF ? 896 : emax - 1023 - kDfTop;
@@ -826,10 +866,11 @@ __device__ __forceinline__ void d2hl(double d, unsigned sub, int thr,
 __device__ __forceinline__ double hl2d(float h, float l, int bias) {
   const unsigned u = (unsigned)__float_as_int(h);
   const unsigned eb = u & 0x7F800000u;
-  // +-2^(52 - e): one unit of the result's last place is 2^(e - 52)
+  // +-2^(52 - e) in two factors (either alone could leave float's range):
+  // one unit of the result's last place is 2^(e - 52)
   const float w =
-      __int_as_float((int)(((306u << 23) - eb) | (u & 0x80000000u)));
-  int n = __float2int_rn(l * w);
+      __int_as_float((int)(((282u << 23) - eb) | (u & 0x80000000u)));
+  int n = __float2int_rn((l * 16777216.f) * w);
   // below a power of two the spacing halves
   if ((u & 0x007FFFFFu) == 0u && n < 0) n += n;
   const unsigned hi = ((unsigned)((int)u >> 3) & 0x8FFFFFFFu) + (unsigned)bias;

@@ -65,3 +65,14 @@ def test_non_finite_stay_in_their_vectors(kind, bad):
         hit.reshape(128, 32, 3)[:, 7, 1] = True
     assert np.abs(y - r)[~hit].max() <= 1e-12 * np.abs(r).max()
     assert not np.isfinite(y[hit]).any()
+
+
+@pytest.mark.parametrize('mag', [1e-30, 1e-24, 1e-10, 1e10, 1e24, 1e32])
+def test_operator_magnitudes(mag):
+    import fastmat_gb300 as fm
+    rng = np.random.default_rng(5)
+    c = rng.standard_normal(128) + 1j * rng.standard_normal(128)
+    x = rng.standard_normal((128, 4)) + 1j * rng.standard_normal((128, 4))
+    y = fm.Circulant(c * mag).forward(np.asfortranarray(x)) / mag
+    r = np.fft.ifft(np.fft.fft(c)[:, None] * np.fft.fft(x, axis=0), axis=0)
+    assert np.abs(y - r).max() <= 1e-12 * np.abs(r).max()
