@@ -208,12 +208,14 @@ class Plan:
         self.handle = handle
         self.compute_type = compute_type
         self._lib = lib
+        self._execute = lib.fm_execute
 
     def execute(self, direction, x_ptr, x_type, ld_x, y_ptr, y_type, ld_y,
                 num_cols, stream):
-        check(self._lib.fm_execute(self.handle, direction, x_ptr, x_type,
-                                   ld_x, y_ptr, y_type, ld_y, num_cols,
-                                   stream))
+        st = self._execute(self.handle, direction, x_ptr, x_type, ld_x,
+                           y_ptr, y_type, ld_y, num_cols, stream)
+        if st:
+            check(st)
 
     def execute_profiled(self, direction, x_ptr, x_type, ld_x, y_ptr, y_type,
                          ld_y, num_cols, stream):

@@ -50,14 +50,9 @@ import numpy as np
 from . import _native
 from . import types as T
 from .matrix import (Conjugate, Hermitian, Matrix, Transpose, _numpy_dtype,
-                     _torch_dtype)
+                     _raw_stream, _torch)
 from .operators import (Circulant, Diag, Eye, Fourier, Kron, Partial,
                         Product, Sum, Toeplitz)
-
-
-def _torch():
-    import torch
-    return torch
 
 
 # ---------------------------------------------------------------- tree
@@ -181,7 +176,7 @@ def _reduce(u, v, pre, n, post, d=None, w=None):
         v = _fcontig(v.to(u.dtype))
     code = _native.DTYPE_CODE[_numpy_dtype(u.dtype)]
     out = torch.empty(n, dtype=u.dtype, device=u.device)
-    stream = torch.cuda.current_stream(u.device).cuda_stream
+    stream = _raw_stream(u.get_device())
     dp = wp = None
     ldw = 0
     if d is not None:
@@ -533,10 +528,10 @@ def _function():
 
         @staticmethod
         def forward(ctx, module, x, *params):
-            prog = module._program()
+            prog = module._program(params)
             x2 = x if x.dim() == 2 else x.unsqueeze(1)
             y, acts = prog.forward(x2)
-            want = _torch_dtype(prog.op._output_dtype(_numpy_dtype(x.dtype)))
+            want = prog.op._io_types(x.dtype)[1]
             if y.dtype != want:
                 y = y.to(want)
             ctx.prog = prog
@@ -630,14 +625,17 @@ class Operator(_module_base()):
         """The wrapped operator with the current parameter values."""
         return self._program().op
 
-    def _key(self):
-        return tuple((p.data_ptr(), p._version) for p in self.parameters())
+    def _key(self, params=None):
+        if params is None:
+            params = self.parameters()
+        return tuple((p.data_ptr(), p._version) for p in params)
 
-    def _program(self):
-        key = self._key()
+    def _program(self, params=None):
+        if params is None:
+            params = list(self.parameters())
+        key = self._key(params)
         if self._prog is not None and key == self._built_key:
             return self._prog
-        params = list(self.parameters())
         if self._prog is None and key == self._values_key:
             op, mapping = self._op, {i: i for i in self._leaf_ids}
         else:

@@ -3066,6 +3066,7 @@ struct HostStage {
   size_t dx_cap = 0, dy_cap = 0;
   cudaStream_t comp = nullptr, in = nullptr, out = nullptr;
   std::vector<cudaEvent_t> ev;  // chunk hand-over events
+  int *status = nullptr;  // page-locked copy of a plan's status word
   void reserve(size_t bx, size_t by) {
     if (bx > dx_cap) {
       if (dx) cudaFree(dx);
@@ -3231,12 +3232,41 @@ int fm_execute_host(fm_plan *plan, int32_t direction, const void *x,
     for (cudaStream_t *sp : {&hs.comp, &hs.in, &hs.out})
       if (!*sp) CUDA_TRY(cudaStreamCreateWithFlags(sp, cudaStreamNonBlocking));
     hs.reserve(bx, by);
+    if (!hs.status)
+      CUDA_TRY(cudaHostAlloc((void **)&hs.status, sizeof(int),
+                             cudaHostAllocDefault));
     // column chunks of at least ~64 MiB of operands, at most 8
     const i64 want = (i64)std::min<size_t>(
         8, std::max<size_t>(1, (bx + by) / ((size_t)64 << 20)));
     const i64 per = (num_cols + std::min<i64>(want, num_cols) - 1) /
                     std::min<i64>(want, num_cols);
     const i64 nch = (num_cols + per - 1) / per;
+    // (the chunks run their fused pairs as separate launches: with the
+    // fused launches inside this pipeline the Kron call measured 19.8
+    // against 7.4 ms)
+    struct NoPair {  // reset also when run_plan throws
+      fm_plan *p;
+      explicit NoPair(fm_plan *q) : p(q) { p->no_pair = true; }
+      ~NoPair() { p->no_pair = false; }
+    } no_pair(plan);
+    if (nch == 1) {
+      // nothing to overlap: one stream in order, the status word read back
+      // with the result, one synchronisation (three streams with hand-over
+      // events and a separate status read cost about 20 us more a call)
+      CUDA_TRY(cudaMemcpyAsync(hs.dx, x, bx, cudaMemcpyHostToDevice,
+                               hs.comp));
+      const int s1 = run_plan(plan, direction, hs.dx, x_type, ld_x, hs.dy,
+                              y_type, ld_y, num_cols, hs.comp);
+      if (s1 != FM_OK) return s1;
+      *hs.status = 0;
+      if (plan->err)
+        CUDA_TRY(cudaMemcpyAsync(hs.status, plan->err, sizeof(int),
+                                 cudaMemcpyDeviceToHost, hs.comp));
+      CUDA_TRY(cudaMemcpyAsync(y, hs.dy, by, cudaMemcpyDeviceToHost,
+                               hs.comp));
+      CUDA_TRY(cudaStreamSynchronize(hs.comp));
+      return *hs.status ? check_status(plan) : (int)FM_OK;
+    }
     while ((i64)hs.ev.size() < 2 * nch) {
       cudaEvent_t e;
       CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -3252,14 +3282,6 @@ int fm_execute_host(fm_plan *plan, int32_t direction, const void *x,
                                cudaMemcpyHostToDevice, hs.in));
       CUDA_TRY(cudaEventRecord(ev_in, hs.in));
       CUDA_TRY(cudaStreamWaitEvent(hs.comp, ev_in, 0));
-      // (the chunks run their fused pairs as separate launches: with the
-      // fused launches inside this pipeline the Kron call measured 19.8
-      // against 7.4 ms)
-      struct NoPair {  // reset also when run_plan throws
-        fm_plan *p;
-        explicit NoPair(fm_plan *q) : p(q) { p->no_pair = true; }
-        ~NoPair() { p->no_pair = false; }
-      } no_pair(plan);
       const int s2 = run_plan(plan, direction, dxk, x_type, ld_x, dyk, y_type,
                               ld_y, m, hs.comp);
       if (s2 != FM_OK) return s2;

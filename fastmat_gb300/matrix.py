@@ -59,38 +59,53 @@ class _Builder:
         return len(self.nodes) - 1
 
 
-_TORCH_DTYPES = None
+_TORCH_DTYPES = None   # numpy dtype -> torch dtype
+_NUMPY_DTYPES = None   # torch dtype -> numpy dtype
+_torch_module = None
 
 
 def _torch():
-    import torch
-    return torch
+    global _torch_module
+    if _torch_module is None:
+        import torch
+        _torch_module = torch
+    return _torch_module
+
+
+def _dtype_tables():
+    global _TORCH_DTYPES, _NUMPY_DTYPES
+    torch = _torch()
+    _NUMPY_DTYPES = {
+        getattr(torch, k): np.dtype(k)
+        for k in ('int8', 'int16', 'int32', 'int64', 'float32', 'float64',
+                  'complex64', 'complex128')}
+    _TORCH_DTYPES = {v: k for k, v in _NUMPY_DTYPES.items()}
 
 
 def _torch_dtype(dt):
-    global _TORCH_DTYPES
-    torch = _torch()
     if _TORCH_DTYPES is None:
-        _TORCH_DTYPES = {
-            np.dtype(np.int8): torch.int8, np.dtype(np.int16): torch.int16,
-            np.dtype(np.int32): torch.int32, np.dtype(np.int64): torch.int64,
-            np.dtype(np.float32): torch.float32,
-            np.dtype(np.float64): torch.float64,
-            np.dtype(np.complex64): torch.complex64,
-            np.dtype(np.complex128): torch.complex128}
+        _dtype_tables()
     return _TORCH_DTYPES[np.dtype(dt)]
 
 
 def _numpy_dtype(tdt):
+    if _NUMPY_DTYPES is None:
+        _dtype_tables()
+    dt = _NUMPY_DTYPES.get(tdt)
+    if dt is None:
+        raise TypeError("unsupported tensor dtype %s" % tdt)
+    return dt
+
+
+def _raw_stream(dev):
+    """Handle of torch's current stream on CUDA device `dev`.  The stream
+    object torch builds for the public call costs several microseconds a
+    call, the raw handle a fraction of one."""
     torch = _torch()
-    for k, v in {np.int8: torch.int8, np.int16: torch.int16,
-                 np.int32: torch.int32, np.int64: torch.int64,
-                 np.float32: torch.float32, np.float64: torch.float64,
-                 np.complex64: torch.complex64,
-                 np.complex128: torch.complex128}.items():
-        if v == tdt:
-            return np.dtype(k)
-    raise TypeError("unsupported tensor dtype %s" % tdt)
+    raw = getattr(torch._C, '_cuda_getCurrentRawStream', None)
+    if raw is not None:
+        return raw(dev)
+    return torch.cuda.current_stream(dev).cuda_stream
 
 
 #: outputs at least this large come from page-locked host memory
@@ -204,6 +219,7 @@ class Matrix:
                 "precision must be 'native', 'fp64', 'fp32' or 'bf16'")
         self._precision = prec
         self._plans = {}
+        self._io = {}   # tensor dtype -> _io_types()
 
     def _getProperties(self):
         return {'minType': self._minType, 'precision': self._precision}
@@ -321,6 +337,22 @@ class Matrix:
             out = T.single(out)
         return out
 
+    def _io_types(self, tdt):
+        """What a tensor of torch dtype `tdt` is transformed as: (its
+        element code, the output's torch dtype and code, numpy output type,
+        the plan's compute code).  It depends on the operator's type and
+        options alone, which do not change, so it is worked out once per
+        tensor dtype."""
+        io = self._io.get(tdt)
+        if io is None:
+            in_dt = _numpy_dtype(tdt)
+            out_dt = np.dtype(self._output_dtype(in_dt))
+            io = self._io[tdt] = (
+                _native.DTYPE_CODE[in_dt], _torch_dtype(out_dt),
+                _native.DTYPE_CODE[out_dt], out_dt,
+                _compute_code(out_dt, self._precision))
+        return io
+
     def plan(self, out_dtype=np.complex128, device=None):
         """The native plan computing in the type of ``out_dtype`` on a CUDA
         device (default: the current one).  A plan's constants live on the
@@ -403,40 +435,56 @@ class Matrix:
         return y.reshape(n_out) if flat else y
 
     def _transform_device(self, x, direction):
+        # (on small operators this call is bound by its own host work: torch
+        # attributes are read once, types and plan looked up, and no stream
+        # or device objects are built when the tensor's device is current)
         torch = _torch()
-        n_req = self.numCols if direction == _native.FORWARD else self.numRows
-        n_out = self.numRows if direction == _native.FORWARD else self.numCols
+        if direction == _native.FORWARD:
+            n_out, n_req = self._shape
+        else:
+            n_req, n_out = self._shape
         if not x.is_cuda:
             return torch.from_numpy(np.ascontiguousarray(
                 self._transform(x.numpy(), direction)))
-        if x.dim() < 1 or x.dim() > 2:
+        shape = x.shape
+        flat = len(shape) == 1
+        if len(shape) < 1 or len(shape) > 2:
             raise ValueError("Input data array must be 1D or 2D")
-        if x.shape[0] != n_req:
+        if shape[0] != n_req:
             raise ValueError(
                 "Mismatch of vector size %d to relevant matrix axis %d" % (
-                    x.shape[0], n_req))
-        flat = x.dim() == 1
-        M = 1 if flat else x.shape[1]
-        in_dt = _numpy_dtype(x.dtype)
-        out_dt = np.dtype(self._output_dtype(in_dt))
+                    shape[0], n_req))
+        M = 1 if flat else shape[1]
+        in_code, out_tdt, out_code, out_dt, code = self._io_types(x.dtype)
+        ld_x = n_req
         if flat:
             xc = x.contiguous()
-        elif x.stride(0) == 1 and (M == 1 or x.stride(1) >= n_req):
-            xc = x
         else:
-            xc = x.t().contiguous().t()
-        # one column: its stride along the (size-1) column axis is irrelevant
-        ld_x = n_req if (flat or M == 1) else xc.stride(1)
-        yt = torch.empty((M, n_out), dtype=_torch_dtype(out_dt),
-                         device=x.device)
+            s0, s1 = x.stride()
+            if s0 == 1 and (M == 1 or s1 >= n_req):
+                xc = x
+                # one column: its stride along the (size-1) column axis is
+                # irrelevant
+                if M != 1:
+                    ld_x = s1
+            else:
+                xc = x.t().contiguous().t()
+        yt = torch.empty((M, n_out), dtype=out_tdt, device=x.device)
         if M > 0:
             # the plan of the tensor's device, launched with it current
-            plan = self.plan(out_dt, device=x.device)
-            with torch.cuda.device(x.device):
-                stream = torch.cuda.current_stream().cuda_stream
-                plan.execute(direction, xc.data_ptr(),
-                             _native.DTYPE_CODE[in_dt], ld_x, yt.data_ptr(),
-                             _native.DTYPE_CODE[out_dt], n_out, M, stream)
+            dev = x.get_device()
+            plan = self._plans.get((dev, code))
+            if plan is None:
+                plan = self.plan(out_dt, device=x.device)
+            if dev == torch.cuda.current_device():
+                plan.execute(direction, xc.data_ptr(), in_code, ld_x,
+                             yt.data_ptr(), out_code, n_out, M,
+                             _raw_stream(dev))
+            else:
+                with torch.cuda.device(dev):
+                    plan.execute(direction, xc.data_ptr(), in_code, ld_x,
+                                 yt.data_ptr(), out_code, n_out, M,
+                                 _raw_stream(dev))
         return yt.reshape(n_out) if flat else yt.t()
 
     # ------------------------------------------------------------ callers
