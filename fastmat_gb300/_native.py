@@ -79,7 +79,7 @@ EXPORTS = ('fm_plan_create', 'fm_execute', 'fm_execute_profiled',
            'fm_plan_destroy', 'fm_plan_get_info', 'fm_plan_describe',
            'fm_batch_create', 'fm_batch_execute', 'fm_batch_execute_graph',
            'fm_batch_check', 'fm_batch_set_wait_limit', 'fm_batch_get_info',
-           'fm_batch_destroy', 'fm_reduce_mulconj',
+           'fm_batch_destroy', 'fm_reduce_mulconj', 'fm_shrink_step',
            'fm_debug_fail_allocation', 'fm_last_error', 'fm_version')
 
 _lib = None
@@ -168,6 +168,10 @@ def load(build_if_missing=True):
                                           P, I64, P, ctypes.c_double, P, P,
                                           I64, P]
         lib.fm_reduce_mulconj.restype = ctypes.c_int
+        D = ctypes.c_double
+        lib.fm_shrink_step.argtypes = [I64, I32, P, P, P, P, P, P, D, D, D,
+                                       P]
+        lib.fm_shrink_step.restype = ctypes.c_int
         lib.fm_last_error.argtypes = []
         lib.fm_last_error.restype = ctypes.c_char_p
         lib.fm_version.argtypes = []
@@ -310,6 +314,14 @@ def reduce_mulconj(A, n, Cc, num_cols, type_code, u, ld_u, v, ld_v, out,
     lib = load()
     check(lib.fm_reduce_mulconj(A, n, Cc, num_cols, type_code, u, ld_u, v,
                                 ld_v, out, scale, d, w, ld_w, stream))
+
+
+def shrink_step(count, type_code, y, g, xold, step, x, ynew, l, alpha, beta,
+                stream=None):
+    """fm_shrink_step on device pointers (see include/fmgpu.h)."""
+    lib = load()
+    check(lib.fm_shrink_step(count, type_code, y, g, xold, step, x, ynew, l,
+                             alpha, beta, stream))
 
 
 class BatchHandle:

@@ -12,9 +12,13 @@ copied to the GPU once and the result copied back once.  The step size
 svds over GPU matvecs, as fastmat/Matrix.pyx:895-921).
 """
 
+import numbers
+
 import numpy as np
 
-from .matrix import Matrix, _torch
+from . import _native
+from .matrix import (Matrix, _device_scope, _numpy_dtype, _raw_stream,
+                     _torch)
 
 
 class _Iterative:
@@ -43,6 +47,50 @@ class _Iterative:
         torch = _torch()
         arrM = torch.clamp(arrX.abs() - numAlpha, min=0)
         return (arrM / (arrM + numAlpha)) * arrX
+
+    def _residual(self, arrB, arrY):
+        """A y - b (in place on the fresh product where that keeps its
+        type)."""
+        r = self.fmatA.forward(arrY)
+        if (r.dtype == arrB.dtype and r.shape == arrB.shape and
+                not arrB.requires_grad):
+            return r.sub_(arrB)
+        return r - arrB
+
+    def _shrink(self, arrY, arrG, numAlpha, arrXold=None, beta=0.0):
+        """(step, x, y) of one iteration: step = y - L g, x its soft
+        threshold, y = x + beta (x - xold) (None without arrXold).  Column-
+        major CUDA tensors of one type take the fused kernel (one launch),
+        anything else separate tensor operations."""
+        torch = _torch()
+        arrs = [arrY, arrG] + ([] if arrXold is None else [arrXold])
+        if (type(self).softThreshold is _Iterative.softThreshold and
+                isinstance(numAlpha, numbers.Real) and
+                isinstance(self.numL, numbers.Real) and
+                arrY.dtype in (torch.float32, torch.float64,
+                               torch.complex64, torch.complex128) and
+                all(a.is_cuda and a.dtype == arrY.dtype and
+                    a.shape == arrY.shape and a.device == arrY.device and
+                    a.t().is_contiguous() and not a.requires_grad and
+                    not a.is_conj() for a in arrs)):
+            step, x = torch.empty_like(arrY), torch.empty_like(arrY)
+            y = None if arrXold is None else torch.empty_like(arrY)
+            dev = arrY.get_device()
+            with _device_scope(-1 if dev == torch.cuda.current_device()
+                               else dev):
+                _native.shrink_step(
+                    arrY.numel(),
+                    _native.DTYPE_CODE[_numpy_dtype(arrY.dtype)],
+                    arrY.data_ptr(), arrG.data_ptr(),
+                    None if arrXold is None else arrXold.data_ptr(),
+                    step.data_ptr(), x.data_ptr(),
+                    None if y is None else y.data_ptr(), self.numL, numAlpha,
+                    beta, _raw_stream(dev))
+            return step, x, y
+        step = arrY - self.numL * arrG
+        x = self.softThreshold(step, numAlpha)
+        return step, x, (None if arrXold is None
+                         else x + beta * (x - arrXold))
 
     def process(self, arrB):
         """Solve for every column of arrB (numpy array or CUDA tensor; the
@@ -84,10 +132,9 @@ class ISTA(_Iterative):
                                 device=arrB.device).t()
         self.arrB = arrB
         for self.numStep in range(self.numMaxSteps):
-            r = A.forward(self.arrX) - arrB
-            self.arrStep = self.arrX - self.numL * A.backward(r)
-            self.arrX = self.softThreshold(
-                self.arrStep, self.numL * self.numLambda * 0.5)
+            r = self._residual(arrB, self.arrX)
+            self.arrStep, self.arrX, _ = self._shrink(
+                self.arrX, A.backward(r), self.numL * self.numLambda * 0.5)
             self.handleCallback(self.cbStep)
             self.handleCallback(self.cbTrace)
         self.arrResult = torch.where(self.arrX != 0, self.arrStep, self.arrX)
@@ -110,14 +157,12 @@ class FISTA(_Iterative):
         self.arrB = arrB
         for self.numStep in range(self.numMaxSteps):
             self.arrXold = self.arrX
-            r = A.forward(self.arrY) - arrB
-            self.arrStep = self.arrY - self.numL * A.backward(r)
-            self.arrX = self.softThreshold(
-                self.arrStep, self.numL * self.numLambda * 0.5)
+            r = self._residual(arrB, self.arrY)
             tOld = self.t
             self.t = (1 + np.sqrt(1 + 4 * self.t ** 2)) / 2
-            self.arrY = self.arrX + ((tOld - 1) / self.t) * (
-                self.arrX - self.arrXold)
+            self.arrStep, self.arrX, self.arrY = self._shrink(
+                self.arrY, A.backward(r), self.numL * self.numLambda * 0.5,
+                self.arrXold, (tOld - 1) / self.t)
             self.handleCallback(self.cbStep)
             self.handleCallback(self.cbTrace)
         return torch.where(self.arrX != 0, self.arrStep, self.arrX)

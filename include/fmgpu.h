@@ -346,6 +346,19 @@ int fm_reduce_mulconj(int64_t A, int64_t n, int64_t Cc, int64_t num_cols,
                       const void *v, int64_t ld_v, void *out, double scale,
                       const void *d, void *w, int64_t ld_w, void *stream);
 
+/* One step of iterative soft thresholding over `count` elements of device
+ * arrays of one type (FM_F32, FM_F64, FM_C64, FM_C128), the elementwise part
+ * of an ISTA / FISTA iteration (fastmat/algorithms/ISTA.py:111-160,
+ * fastmat/algorithms/FISTA.py:120-180):
+ *
+ *   step = y - l g;  x = m / (m + alpha) step, m = max(|step| - alpha, 0);
+ *   ynew = x + beta (x - xold)      (skipped when ynew is NULL)
+ *
+ * step, x and ynew must not overlap the inputs or one another. */
+int fm_shrink_step(int64_t count, int32_t type, const void *y, const void *g,
+                   const void *xold, void *step, void *x, void *ynew,
+                   double l, double alpha, double beta, void *stream);
+
 /* Test hook for the out-of-memory path: after `after` more device
  * allocations of this library succeed, the next one fails as if the device
  * were full (the call then returns FM_ERR_NOMEM and frees what it had
