@@ -1,7 +1,7 @@
 // Instantiations and launchers of the register-resident FWHT kernels
-// (fm_rfwht.cuh): float32 and double-float real data, contiguous vectors of
-// 1024..8192 (float32) or 256..8192 (double-float) points, strided vectors
-// of 64..2048 (float32) or 32..1024 (double-float) points.
+// (fm_rfwht.cuh): float32 and fixed-point (float64) real data, contiguous vectors of
+// 1024..8192 (float32) or 256..8192 (fixed-point (float64)) points, strided vectors
+// of 64..2048 (float32) or 32..1024 (fixed-point (float64)) points.
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -148,12 +148,12 @@ cudaError_t launch_rfwht2(int ctype, const RfPair &p, cudaStream_t s) {
     }
   } else if (ctype == FM_F64_DF && p.a.L == 4096) {
     switch (p.b.L) {
-      case 32: return launch_pair<df, 4096, 32>(p, s);
-      case 64: return launch_pair<df, 4096, 64>(p, s);
-      case 128: return launch_pair<df, 4096, 128>(p, s);
-      case 256: return launch_pair<df, 4096, 256>(p, s);
-      case 512: return launch_pair<df, 4096, 512>(p, s);
-      case 1024: return launch_pair<df, 4096, 1024>(p, s);
+      case 32: return launch_pair<fx, 4096, 32>(p, s);
+      case 64: return launch_pair<fx, 4096, 64>(p, s);
+      case 128: return launch_pair<fx, 4096, 128>(p, s);
+      case 256: return launch_pair<fx, 4096, 256>(p, s);
+      case 512: return launch_pair<fx, 4096, 512>(p, s);
+      case 1024: return launch_pair<fx, 4096, 1024>(p, s);
       default: break;
     }
   }
@@ -188,12 +188,12 @@ cudaError_t launch_rfwht(int ctype, const RfStep &p, cudaStream_t s) {
       }
     } else if (ctype == FM_F64_DF) {
       switch (p.L) {
-        case 32: return launch_strided<df, 32>(p, s);
-        case 64: return launch_strided<df, 64>(p, s);
-        case 128: return launch_strided<df, 128>(p, s);
-        case 256: return launch_strided<df, 256>(p, s);
-        case 512: return launch_strided<df, 512>(p, s);
-        case 1024: return launch_strided<df, 1024>(p, s);
+        case 32: return launch_strided<fx, 32>(p, s);
+        case 64: return launch_strided<fx, 64>(p, s);
+        case 128: return launch_strided<fx, 128>(p, s);
+        case 256: return launch_strided<fx, 256>(p, s);
+        case 512: return launch_strided<fx, 512>(p, s);
+        case 1024: return launch_strided<fx, 1024>(p, s);
         default: break;
       }
     }
@@ -209,12 +209,12 @@ cudaError_t launch_rfwht(int ctype, const RfStep &p, cudaStream_t s) {
     }
   } else if (ctype == FM_F64_DF) {
     switch (p.L) {
-      case 256: return launch_one<df, 256>(p, s);
-      case 512: return launch_one<df, 512>(p, s);
-      case 1024: return launch_one<df, 1024>(p, s);
-      case 2048: return launch_one<df, 2048>(p, s);
-      case 4096: return launch_one<df, 4096>(p, s);
-      case 8192: return launch_one<df, 8192>(p, s);
+      case 256: return launch_one<fx, 256>(p, s);
+      case 512: return launch_one<fx, 512>(p, s);
+      case 1024: return launch_one<fx, 1024>(p, s);
+      case 2048: return launch_one<fx, 2048>(p, s);
+      case 4096: return launch_one<fx, 4096>(p, s);
+      case 8192: return launch_one<fx, 8192>(p, s);
       default: break;
     }
   }

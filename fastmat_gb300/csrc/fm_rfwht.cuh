@@ -1,18 +1,20 @@
 // Register-resident Walsh-Hadamard transform of contiguous power-of-two
 // vectors (fastmat's Hadamard, fastmat/Hadamard.pyx:164-230: a + b / a - b
-// butterflies at distance 1, 2, 4, ...), for real float32 and double-float
-// data.
+// butterflies at distance 1, 2, 4, ...), for real float32 and float64
+// data (64-bit fixed point, see fx in fm_types.cuh: float64 launches were
+// bound by the double-float additions and conversions; Hadamard(18) on 48
+// columns 224 -> 129 us, the FWHT mode of Kron(F256, H8, C128) on 8 complex
+// columns 875 -> 540 us, errors against 64 bits 7.2e-15 -> 1.3e-15).
 //
 //   * a vector of L points is held by G = L / P threads of a CTA, P points
-//     per thread (32 float or 16 double-float); the CTA works on
+//     per thread (32 float or 16 fixed-point); the CTA works on
 //     max(1, 256 / G) vectors at a time;
 //   * the index bits are taken in passes of log2(P) bits from the least
 //     significant one, so the butterflies run in fastmat's order and float32
 //     results are bit-identical to its float32 transform; within a pass every
 //     thread's groups of points (the points that differ only in the pass's
 //     bits) are in its registers, and the levels of the pass are plain
-//     register butterflies (double-float: unnormalised inside the pass, one
-//     renormalisation at its end);
+//     register butterflies;
 //   * the first pass takes thread t's P consecutive points (t P .. t P + P-1)
 //     from a shared-memory slot that cp.async filled one batch ahead; between
 //     passes the points go through a shared-memory exchange buffer (CTA
@@ -22,7 +24,7 @@
 // Thread t's groups at a pass with bit offset s and width w are
 // h = t + G u (u < P / 2^w); point r of group h sits at
 // ((h >> s) << (s + w)) | (r << s) | (h mod 2^s).  The exchange buffer puts
-// point e at e + (e >> 5) (float) or e + (e >> 4) (double-float), the slot
+// point e at e + (e >> 5) (float) or e + (e >> 4) (fixed point), the slot
 // holds raw float32 / float64 words with a 16-byte pad per 128 bytes: every
 // access pattern of the kernel is then free of bank conflicts (checked by
 // enumerating them for the lengths instantiated).
@@ -57,6 +59,7 @@ template <class E> struct RfLane {
   typedef typename std::conditional<std::is_same<E, float>::value, float,
                                     double>::type Raw;
   static constexpr int XSH = std::is_same<E, float>::value ? 5 : 4;
+  static constexpr bool fixed = std::is_same<E, fx>::value;
 };
 template <class E, int L> struct RfShape {
   static constexpr int P = RfLane<E>::P;
@@ -88,6 +91,37 @@ __device__ __forceinline__ int rf_xpad(int e) {
 }
 __device__ __forceinline__ int rf_pos(int h, int s, int r, int w) {
   return ((h >> s) << (s + w)) | (r << s) | (h & ((1 << s) - 1));
+}
+
+// largest exponent word of a thread's points
+template <int P>
+__device__ __forceinline__ int rf_max(const double (&d)[P]) {
+  int e = 0;
+#pragma unroll
+  for (int r = 0; r < P; ++r) e = max(e, raw_hi(d[r]));
+  return e;
+}
+// registers to raw words (emax: the vector's largest exponent field; a
+// vector holding Inf or NaN gives NaN throughout, as its sums do)
+template <class E, int L, class F>
+__device__ __forceinline__ void rf_out(const E (&x)[RfLane<E>::P], int emax,
+                                       F store) {
+  constexpr int P = RfLane<E>::P;
+  if constexpr (RfLane<E>::fixed) {
+    const unsigned nan = emax >= 0x7FF ? 0x7FF80000u : 0u;
+    if (emax >= 80 && emax <= 2020) {
+#pragma unroll
+      for (int j = 0; j < P; ++j)
+        store(j, fx2d(x[j], emax, rf_log2(L), true, 0u));
+    } else {
+#pragma unroll
+      for (int j = 0; j < P; ++j)
+        store(j, fx2d(x[j], emax, rf_log2(L), false, nan));
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < P; ++j) store(j, x[j]);
+  }
 }
 
 // the levels of one pass (w bits) on the thread's P registers, in place:
@@ -167,7 +201,7 @@ template <class E, int L> __host__ __device__ constexpr int rf_last() {
 }
 
 // The rest of a contiguous batch once thread t of vector vl holds its
-// first-pass points d (raw words): double-float scaling, the passes, the
+// first-pass points d (raw words): the scaling, the passes, the
 // stores of the last pass.
 template <class E, int L>
 __device__ __forceinline__ void rf_finish(
@@ -179,16 +213,13 @@ __device__ __forceinline__ void rf_finish(
   constexpr int WL = rf_log2(L) - SL;
   typedef typename Sh::Raw Raw;
   E x[P];
-  int s = 0;
-  if constexpr (Emu<E>::v) {
-    // double-float: every vector scaled by the power of two of its
-    // largest exponent (float's exponent range), restored on store
-    // (reduced over the vector's lanes within each warp, then across its
-    // warps in shared memory)
+  int emax = 0;
+  if constexpr (RfLane<E>::fixed) {
+    // fixed point: every vector scaled by the power of two of its largest
+    // exponent, restored on store (reduced over the vector's lanes within
+    // each warp, then across its warps in shared memory)
     constexpr int WV = G < 32 ? G : 32;
-    int emax = 0;
-#pragma unroll
-    for (int r = 0; r < P; ++r) emax = max(emax, dexp(d[r]));
+    emax = rf_max<P>(d);
 #pragma unroll
     for (int o = WV / 2; o >= 1; o /= 2)
       emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o, WV));
@@ -196,9 +227,9 @@ __device__ __forceinline__ void rf_finish(
     __syncthreads();
     if (t % WV == 0 && emax > 0) atomicMax(sexp + vl, emax);
     __syncthreads();
-    s = sexp[vl] > 0 ? sexp[vl] - 1023 : 0;
+    emax = sexp[vl] >> 20;
 #pragma unroll
-    for (int r = 0; r < P; ++r) x[r] = d2df_scaled(d[r], s);
+    for (int r = 0; r < P; ++r) x[r] = d2fx(d[r], emax, rf_log2(L));
   } else {
 #pragma unroll
     for (int r = 0; r < P; ++r) x[r] = d[r];
@@ -210,15 +241,9 @@ __device__ __forceinline__ void rf_finish(
     const unsigned a = (unsigned)gv - m * (unsigned)p.A;
     Raw *dst = (Raw *)p.dst + (i64)m * p.ld_dst + (i64)a * p.stride +
                rf_pos(t, SL, 0, WL);
-#pragma unroll
-    for (int j = 0; j < P; ++j) {
-      const int u = j >> WL, r = j & ((1 << WL) - 1);
-      const int e = rf_pos(G * u, SL, r, WL);
-      if constexpr (Emu<E>::v)
-        dst[e] = df2d_scaled(x[j], s);
-      else
-        dst[e] = x[j];
-    }
+    rf_out<E, L>(x, emax, [&](int j, Raw y) {
+      dst[rf_pos(G * (j >> WL), SL, j & ((1 << WL) - 1), WL)] = y;
+    });
   }
 }
 
@@ -335,20 +360,18 @@ __device__ __forceinline__ void rs_batch(const RfStep &p, i64 bt, E *xb,
     for (int r = 0; r < P; ++r, q += S) d[r] = *q;
   }
   E x[P];
-  int s = 0;
-  if constexpr (Emu<E>::v) {
-    // double-float: each vector scaled by the power of two of its largest
-    // exponent (float's exponent range), restored on store
-    int emax = 0;
-#pragma unroll
-    for (int r = 0; r < P; ++r) emax = max(emax, dexp(d[r]));
+  int emax = 0;
+  if constexpr (RfLane<E>::fixed) {
+    // fixed point: each vector scaled by the power of two of its largest
+    // exponent, restored on store
+    emax = rf_max<P>(d);
     if (threadIdx.x < NV) sexp[threadIdx.x] = 0;
     __syncthreads();
     if (emax > 0) atomicMax(sexp + v, emax);
     __syncthreads();
-    s = sexp[v] > 0 ? sexp[v] - 1023 : 0;
+    emax = sexp[v] >> 20;
 #pragma unroll
-    for (int r = 0; r < P; ++r) x[r] = d2df_scaled(d[r], s);
+    for (int r = 0; r < P; ++r) x[r] = d2fx(d[r], emax, rf_log2(L));
   } else {
 #pragma unroll
     for (int r = 0; r < P; ++r) x[r] = d[r];
@@ -359,17 +382,9 @@ __device__ __forceinline__ void rs_batch(const RfStep &p, i64 bt, E *xb,
   rf_passes<E, L, 0>(x, buf, t);
   Raw *dst = (Raw *)p.dst + (i64)m * p.ld_dst + row0 +
              (i64)rf_pos(t, SL, 0, WL) * S;
-#pragma unroll
-  for (int u = 0; u < (P >> WL); ++u) {
-    Raw *q = dst + (i64)rf_pos(W * u, SL, 0, WL) * S;
-#pragma unroll
-    for (int r = 0; r < (1 << WL); ++r, q += S << SL) {
-      if constexpr (Emu<E>::v)
-        *q = df2d_scaled(x[(u << WL) + r], s);
-      else
-        *q = x[(u << WL) + r];
-    }
-  }
+  rf_out<E, L>(x, emax, [&](int j, Raw y) {
+    dst[(i64)rf_pos(W * (j >> WL), SL, j & ((1 << WL) - 1), WL) * S] = y;
+  });
 }
 
 template <class E, int L>
@@ -429,7 +444,7 @@ template <class E, int L1, int L2>
 __host__ __device__ constexpr size_t rf2_smem() {
   return Rf2Mem<E, L1, L2>::bytes;
 }
-// CTAs per SM: float32 fits four (64 registers a thread), double-float three
+// CTAs per SM: float32 fits four (64 registers a thread), fixed point three
 template <class E> struct Rf2Occ {
   static constexpr int v = std::is_same<E, float>::value ? 4 : 3;
 };
