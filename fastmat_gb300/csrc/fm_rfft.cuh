@@ -95,19 +95,19 @@ template <class E, int L> struct RxShape {
   static constexpr int Lc = RcBuf<E, L>::Lp;
 };
 // threads per SM the register budget aims at: 128 registers a thread in
-// double-float, 64 in complex64
-template <class E> struct RxTPS {
-  static constexpr int v = sizeof(E) != 8 ? 512 : 1024;
+// double-float; complex64 64 for one FFT, 80 for the convolution
+template <class E, bool CONV> struct RxTPS {
+  static constexpr int v = sizeof(E) != 8 ? 512 : CONV ? 768 : 1024;
 };
 template <class E, int L>
 __host__ __device__ constexpr size_t rxfft_smem() {
   typedef RxShape<E, L> S;
-  return (size_t)S::NV * S::Lx * sizeof(E) + 32 * sizeof(int);
+  return (size_t)2 * S::NV * S::Lx * sizeof(E) + 32 * sizeof(int);
 }
 template <class E, int L>
 __host__ __device__ constexpr size_t rxconv_smem() {
   typedef RxShape<E, L> S;
-  return (size_t)S::VPC * S::Lc * sizeof(E) + S::VPC * sizeof(int);
+  return (size_t)S::VPC * (S::Lc + L) * sizeof(E) + S::VPC * sizeof(int);
 }
 
 template <class E> struct RxRaw {
@@ -169,6 +169,34 @@ __device__ __forceinline__ void rx_load(
   const unsigned m = p.conj_in ? 0x80000000u : 0u;
 #pragma unroll
   for (int r = 0; r < P; ++r) d[r] = rx_conj(d[r], m);
+}
+
+// copy points j0 + dj r of one vector ahead into shared memory (dst + ds r),
+// zeros outside the vector or the column; buffers already in the kernel's
+// type without a gather only
+template <class E, int L>
+__device__ __forceinline__ void rx_ahead(const RxStep &p, bool act, i64 col,
+                                         i64 rb, int j0, int dj,
+                                         typename RxRaw<E>::type *dst,
+                                         int ds) {
+  typedef typename RxRaw<E>::type Raw;
+  constexpr int P = RcLane<E>::P;
+  const i64 cc = p.in_cc;
+  const Raw *q = (const Raw *)p.src + col + rb + (i64)j0 * cc;
+  const i64 step = (i64)dj * cc;
+  if (act && p.in_len == L && rb + (L - 1) * cc < p.in_rows) {
+#pragma unroll
+    for (int r = 0; r < P; ++r)
+      cp_async<sizeof(Raw)>(dst + ds * r, q + r * step, true);
+  } else {
+#pragma unroll
+    for (int r = 0; r < P; ++r) {
+      const int j = j0 + dj * r;
+      const bool ok = act && j < p.in_len && rb + (i64)j * cc < p.in_rows;
+      cp_async<sizeof(Raw)>(dst + ds * r,
+                            ok ? (const void *)(q + r * step) : p.src, ok);
+    }
+  }
 }
 
 // the loader's product on points j0 + dj r
@@ -239,7 +267,7 @@ __device__ __forceinline__ void rx_store(E (&x)[RcLane<E>::P], int s,
 
 template <class E, int L>
 __global__ void __launch_bounds__(RxShape<E, L>::TF,
-                                  RxTPS<E>::v / RxShape<E, L>::TF)
+                                  RxTPS<E, false>::v / RxShape<E, L>::TF)
     rxfft_kernel(const __grid_constant__ RxStep p) {
   typedef RxShape<E, L> Sh;
   typedef typename RxRaw<E>::type Raw;
@@ -249,13 +277,41 @@ __global__ void __launch_bounds__(RxShape<E, L>::TF,
   static_assert(S >= 2 && T <= 512 && T * P == NV * L, "vector layout");
   extern __shared__ __align__(128) unsigned char fm_smem[];
   E *xb = reinterpret_cast<E *>(fm_smem);
-  int *sexp = reinterpret_cast<int *>(xb + NV * Sh::Lx);
+  Raw *slot = reinterpret_cast<Raw *>(xb + NV * Sh::Lx);  // the next batch
+  int *sexp = reinterpret_cast<int *>(slot + NV * Sh::Lx);
   const int lane = threadIdx.x % NV, t = threadIdx.x / NV;
   E *buf = xb + lane * Sh::Lx;
   const unsigned nbc = (unsigned)((p.V + NV - 1) / NV);  // batches per column
   const unsigned nb = nbc * (unsigned)p.num_cols;
   const FDiv dB(nbc), dI((unsigned)p.in_cc), dO((unsigned)p.out_cc);
   const int jn = rc_nat<E, L>(rc_base<E, L, S - 1>(t));
+  // contiguous vectors are loaded along their points (thread k takes point
+  // k + T i of the batch's NV L points) and turned on the way through shared
+  // memory; strided ones by the thread that uses them
+  const bool turn = p.in_cc == 1;
+  const bool ahead = p.src_type == Tr<E>::code && !p.map_in;
+  auto prefetch = [&](unsigned bt) {
+    const unsigned m = dB.div(bt), v0 = (bt - m * nbc) * NV;
+    const i64 col = (i64)m * p.ld_src;
+    if (turn) {
+#pragma unroll
+      for (int i = 0; i < P; ++i) {
+        const int k = threadIdx.x + T * i, vv = k / L, j = k % L;
+        const i64 row = (i64)(v0 + vv) * p.in_n + j;
+        const bool ok = v0 + vv < p.V && j < p.in_len && row < p.in_rows;
+        cp_async<sizeof(Raw)>(
+            slot + vv * Sh::Lx + rc_pad<E, L>(j),
+            ok ? (const void *)((const Raw *)p.src + col + row) : p.src, ok);
+      }
+    } else {
+      const unsigned v = v0 + lane;
+      const unsigned a = dI.div(v), c = v - a * (unsigned)p.in_cc;
+      rx_ahead<E, L>(p, v < p.V, col, (i64)a * p.in_n * p.in_cc + c, t, G,
+                     slot + threadIdx.x, T);
+    }
+    cp_async_commit();
+  };
+  if (ahead && blockIdx.x < nb) prefetch(blockIdx.x);
   for (unsigned bt = blockIdx.x; bt < nb; bt += gridDim.x) {
     const unsigned m = dB.div(bt), v0 = (bt - m * nbc) * NV;
     const unsigned v = v0 + lane;
@@ -264,41 +320,42 @@ __global__ void __launch_bounds__(RxShape<E, L>::TF,
     const i64 rb = (i64)a * p.in_n * p.in_cc + c;
     const i64 col = (i64)m * p.ld_src;
     Raw d[P];
-    if (p.in_cc == 1) {
-      // contiguous vectors: loads along the points, turned through the
-      // exchange buffer (thread k takes point k + T i of the NV L points)
-      Raw *rw = reinterpret_cast<Raw *>(xb);
+    if (turn) {
+      if (ahead) {
+        cp_async_wait<0>();
+      } else {
 #pragma unroll
-      for (int i = 0; i < P; ++i) {
-        const int k = threadIdx.x + T * i, vv = k / L, j = k % L;
-        const i64 rv = (i64)(v0 + vv) * p.in_n;
-        Raw y = rx_zero(Raw());
-        if (v0 + vv < p.V && j < p.in_len && rv + j < p.in_rows) {
-          if (p.src_type == Tr<E>::code && !p.map_in) {
-            y = ((const Raw *)p.src)[col + rv + j];
-          } else {
+        for (int i = 0; i < P; ++i) {
+          const int k = threadIdx.x + T * i, vv = k / L, j = k % L;
+          const i64 rv = (i64)(v0 + vv) * p.in_n;
+          Raw y = rx_zero(Raw());
+          if (v0 + vv < p.V && j < p.in_len && rv + j < p.in_rows) {
             const i64 srow = p.map_in ? p.map_in[rv + j] : rv + j;
             if (srow >= 0) y = load_as<Raw>(p.src, p.src_type, col + srow);
           }
+          slot[vv * Sh::Lx + rc_pad<E, L>(j)] = y;
         }
-        d[i] = rx_conj(y, p.conj_in ? 0x80000000u : 0u);
-      }
-#pragma unroll
-      for (int i = 0; i < P; ++i) {
-        const int k = threadIdx.x + T * i, vv = k / L, j = k % L;
-        rw[vv * Sh::Lx + rc_pad<E, L>(j)] = d[i];
       }
       __syncthreads();
-      const Raw *rr = rw + lane * Sh::Lx + rc_pad<E, L>(t);
+      // (t < G, so t and G r occupy disjoint bits)
+      const Raw *rr = slot + lane * Sh::Lx + rc_pad<E, L>(t);
+      const unsigned mask = p.conj_in ? 0x80000000u : 0u;
 #pragma unroll
-      for (int r = 0; r < P; ++r) {
-        // (t < G, so t and G r occupy disjoint bits)
-        d[r] = rr[rc_pad<E, L>(G * r)];
-      }
+      for (int r = 0; r < P; ++r)
+        d[r] = rx_conj(rr[rc_pad<E, L>(G * r)], mask);
       __syncthreads();
+    } else if (ahead) {
+      cp_async_wait<0>();
+      __syncwarp();
+      const unsigned mask = p.conj_in ? 0x80000000u : 0u;
+#pragma unroll
+      for (int r = 0; r < P; ++r)
+        d[r] = rx_conj(slot[threadIdx.x + T * r], mask);
+      __syncwarp();
     } else {
       rx_load<E, L>(d, p, act, col, rb, t, G);
     }
+    if (ahead && bt + gridDim.x < nb) prefetch(bt + gridDim.x);
     E x[P];
     int s = 0;
     if constexpr (Emu<E>::v) {
@@ -330,7 +387,7 @@ __global__ void __launch_bounds__(RxShape<E, L>::TF,
 
 template <class E, int L>
 __global__ void __launch_bounds__(RxShape<E, L>::TC,
-                                  RxTPS<E>::v / RxShape<E, L>::TC)
+                                  RxTPS<E, true>::v / RxShape<E, L>::TC)
     rxconv_kernel(const __grid_constant__ RxStep p) {
   typedef RxShape<E, L> Sh;
   typedef typename RxRaw<E>::type Raw;
@@ -340,18 +397,41 @@ __global__ void __launch_bounds__(RxShape<E, L>::TC,
   static_assert(S >= 2 && Sh::TC <= 512, "vector layout");
   extern __shared__ __align__(128) unsigned char fm_smem[];
   E *xb = reinterpret_cast<E *>(fm_smem);
-  int *sexp = reinterpret_cast<int *>(xb + VPC * Sh::Lc);
+  Raw *slot = reinterpret_cast<Raw *>(xb + VPC * Sh::Lc) + threadIdx.x;
+  int *sexp = reinterpret_cast<int *>(fm_smem) +
+              VPC * (Sh::Lc + L) * (sizeof(E) / sizeof(int));
   const int q = threadIdx.x / G, g = threadIdx.x % G;
   E *buf = xb + q * Sh::Lc;
   const unsigned NV = (unsigned)(p.V * p.num_cols);
   const FDiv dV((unsigned)p.V);
+  // the next batch's points, copied ahead by the threads that use them
+  const bool ahead = p.src_type == Tr<E>::code && !p.map_in;
+  auto prefetch = [&](unsigned vb) {
+    const unsigned gv = vb + q;
+    const unsigned m = dV.div(gv), v = gv - m * (unsigned)p.V;
+    rx_ahead<E, L>(p, gv < NV, (i64)m * p.ld_src, (i64)v * p.in_n, g, G,
+                   slot, Sh::TC);
+    cp_async_commit();
+  };
+  if (ahead && blockIdx.x * VPC < NV) prefetch(blockIdx.x * VPC);
   for (unsigned vb = blockIdx.x * VPC; vb < NV; vb += gridDim.x * VPC) {
     const unsigned gv = vb + q;
     const bool act = gv < NV;
     const unsigned m = dV.div(gv), v = gv - m * (unsigned)p.V;
     const i64 rb = (i64)v * p.in_n;
     Raw d[P];
-    rx_load<E, L>(d, p, act, (i64)m * p.ld_src, rb, g, G);
+    if (ahead) {
+      cp_async_wait<0>();
+      __syncwarp();
+      const unsigned mask = p.conj_in ? 0x80000000u : 0u;
+#pragma unroll
+      for (int r = 0; r < P; ++r) d[r] = rx_conj(slot[Sh::TC * r], mask);
+      __syncwarp();
+      const unsigned nx = vb + gridDim.x * VPC;
+      if (nx < NV) prefetch(nx);
+    } else {
+      rx_load<E, L>(d, p, act, (i64)m * p.ld_src, rb, g, G);
+    }
     E x[P];
     int s = 0;
     if constexpr (Emu<E>::v) {
