@@ -131,7 +131,7 @@ __device__ __forceinline__ float2 rx_zero(float2) {
 }
 
 // P points j0 + dj r of one vector of the input view (row of point 0: rb,
-// column offset col), zero outside the vector or the column
+// column offset col) from any type, zero outside the vector or the column
 template <class E, int L>
 __device__ __forceinline__ void rx_load(
     typename RxRaw<E>::type (&d)[RcLane<E>::P], const RxStep &p, bool act,
@@ -139,32 +139,16 @@ __device__ __forceinline__ void rx_load(
   typedef typename RxRaw<E>::type Raw;
   constexpr int P = RcLane<E>::P;
   const i64 cc = p.in_cc;
-  if (p.src_type == Tr<E>::code && !p.map_in) {
-    const Raw *q = (const Raw *)p.src + col + rb + (i64)j0 * cc;
-    const i64 step = (i64)dj * cc;
-    if (act && p.in_len == L && rb + (L - 1) * cc < p.in_rows) {
 #pragma unroll
-      for (int r = 0; r < P; ++r) d[r] = q[r * step];
-    } else {
-#pragma unroll
-      for (int r = 0; r < P; ++r) {
-        const int j = j0 + dj * r;
-        const bool ok = act && j < p.in_len && rb + (i64)j * cc < p.in_rows;
-        d[r] = ok ? q[r * step] : rx_zero(Raw());
-      }
+  for (int r = 0; r < P; ++r) {
+    const int j = j0 + dj * r;
+    const i64 row = rb + (i64)j * cc;
+    Raw v = rx_zero(Raw());
+    if (act && j < p.in_len && row < p.in_rows) {
+      const i64 srow = p.map_in ? p.map_in[row] : row;
+      if (srow >= 0) v = load_as<Raw>(p.src, p.src_type, col + srow);
     }
-  } else {
-#pragma unroll
-    for (int r = 0; r < P; ++r) {
-      const int j = j0 + dj * r;
-      const i64 row = rb + (i64)j * cc;
-      Raw v = rx_zero(Raw());
-      if (act && j < p.in_len && row < p.in_rows) {
-        const i64 srow = p.map_in ? p.map_in[row] : row;
-        if (srow >= 0) v = load_as<Raw>(p.src, p.src_type, col + srow);
-      }
-      d[r] = v;
-    }
+    d[r] = v;
   }
   const unsigned m = p.conj_in ? 0x80000000u : 0u;
 #pragma unroll
@@ -172,8 +156,8 @@ __device__ __forceinline__ void rx_load(
 }
 
 // copy points j0 + dj r of one vector ahead into shared memory (dst + ds r),
-// zeros outside the vector or the column; buffers already in the kernel's
-// type without a gather only
+// zeros outside the vector or the column and where the gather has none;
+// buffers already in the kernel's type only
 template <class E, int L>
 __device__ __forceinline__ void rx_ahead(const RxStep &p, bool act, i64 col,
                                          i64 rb, int j0, int dj,
@@ -184,7 +168,22 @@ __device__ __forceinline__ void rx_ahead(const RxStep &p, bool act, i64 col,
   const i64 cc = p.in_cc;
   const Raw *q = (const Raw *)p.src + col + rb + (i64)j0 * cc;
   const i64 step = (i64)dj * cc;
-  if (act && p.in_len == L && rb + (L - 1) * cc < p.in_rows) {
+  if (p.map_in) {
+    i64 row[P];
+#pragma unroll
+    for (int r = 0; r < P; ++r) {
+      const int j = j0 + dj * r;
+      const i64 k = rb + (i64)j * cc;
+      row[r] = act && j < p.in_len && k < p.in_rows ? p.map_in[k] : -1;
+    }
+#pragma unroll
+    for (int r = 0; r < P; ++r)
+      cp_async<sizeof(Raw)>(
+          dst + ds * r,
+          row[r] >= 0 ? (const void *)((const Raw *)p.src + col + row[r])
+                      : p.src,
+          row[r] >= 0);
+  } else if (act && p.in_len == L && rb + (L - 1) * cc < p.in_rows) {
 #pragma unroll
     for (int r = 0; r < P; ++r)
       cp_async<sizeof(Raw)>(dst + ds * r, q + r * step, true);
@@ -230,10 +229,35 @@ __device__ __forceinline__ void rx_store(E (&x)[RcLane<E>::P], int s,
       x[r] = mulv(x[r], f, p.w_conj != 0);
     }
   }
-  if (p.dst_type == Tr<E>::code && !p.accumulate && !p.post &&
-      !p.has_scale && !p.map_out) {
+  if (p.post) {
+#pragma unroll
+    for (int r = 0; r < P; ++r) {
+      const int j = j0 + jo(r);
+      const i64 row = rb + (i64)j * cc;
+      if (j < p.out_len && row < p.out_rows)
+        x[r] = mulv(x[r], tab_get<E>(p.post, p.post_by_point ? (i64)j : row),
+                    p.post_conj != 0);
+    }
+  }
+  if (p.has_scale) {
+    const E c = scalar_of<E>(p.scale_re, p.scale_im);
+#pragma unroll
+    for (int r = 0; r < P; ++r) x[r] = mulv(x[r], c, false);
+  }
+  if (p.dst_type == Tr<E>::code && !p.accumulate) {
     const unsigned m = p.conj_out ? 0x80000000u : 0u;
-    Raw *q = (Raw *)p.dst + col + rb + (i64)j0 * cc;
+    Raw *const dst = (Raw *)p.dst + col;
+    if (p.map_out) {
+      rx_out<P>(x, s, [&](int r, Raw y) {
+        const int j = j0 + jo(r);
+        const i64 row = rb + (i64)j * cc;
+        const i64 drow =
+            j < p.out_len && row < p.out_rows ? p.map_out[row] : -1;
+        if (drow >= 0) dst[drow] = rx_conj(y, m);
+      });
+      return;
+    }
+    Raw *q = dst + rb + (i64)j0 * cc;
     if (p.out_len == L && rb + (L - 1) * cc < p.out_rows) {
       rx_out<P>(x, s, [&](int r, Raw y) {
         q[(i64)jo(r) * cc] = rx_conj(y, m);
@@ -247,7 +271,6 @@ __device__ __forceinline__ void rx_store(E (&x)[RcLane<E>::P], int s,
     }
     return;
   }
-  const E c = scalar_of<E>(p.scale_re, p.scale_im);
 #pragma unroll
   for (int r = 0; r < P; ++r) {
     const int j = j0 + jo(r);
@@ -255,13 +278,8 @@ __device__ __forceinline__ void rx_store(E (&x)[RcLane<E>::P], int s,
     if (j >= p.out_len || row >= p.out_rows) continue;
     const i64 drow = p.map_out ? p.map_out[row] : row;
     if (drow < 0) continue;
-    E y = x[r];
-    if (p.post)
-      y = mulv(y, tab_get<E>(p.post, p.post_by_point ? (i64)j : row),
-               p.post_conj != 0);
-    if (p.has_scale) y = mulv(y, c, false);
-    if (p.conj_out) y = conjv(y);
-    store_elem<E>(p.dst, p.dst_type, col + drow, y, p.accumulate != 0, s);
+    store_elem<E>(p.dst, p.dst_type, col + drow,
+                  p.conj_out ? conjv(x[r]) : x[r], p.accumulate != 0, s);
   }
 }
 
@@ -289,7 +307,7 @@ __global__ void __launch_bounds__(RxShape<E, L>::TF,
   // k + T i of the batch's NV L points) and turned on the way through shared
   // memory; strided ones by the thread that uses them
   const bool turn = p.in_cc == 1;
-  const bool ahead = p.src_type == Tr<E>::code && !p.map_in;
+  const bool ahead = p.src_type == Tr<E>::code && !(turn && p.map_in);
   auto prefetch = [&](unsigned bt) {
     const unsigned m = dB.div(bt), v0 = (bt - m * nbc) * NV;
     const i64 col = (i64)m * p.ld_src;
@@ -405,7 +423,7 @@ __global__ void __launch_bounds__(RxShape<E, L>::TC,
   const unsigned NV = (unsigned)(p.V * p.num_cols);
   const FDiv dV((unsigned)p.V);
   // the next batch's points, copied ahead by the threads that use them
-  const bool ahead = p.src_type == Tr<E>::code && !p.map_in;
+  const bool ahead = p.src_type == Tr<E>::code;
   auto prefetch = [&](unsigned vb) {
     const unsigned gv = vb + q;
     const unsigned m = dV.div(gv), v = gv - m * (unsigned)p.V;
