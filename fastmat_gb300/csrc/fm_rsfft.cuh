@@ -51,10 +51,15 @@ template <class E, int L> struct RsfShape {
 template <class E> struct RsfOcc {
   static constexpr int v = sizeof(E) == 8 ? 3 : 2;
 };
+// double-float copies the next batch ahead into shared memory while the
+// current one transforms (its two CTAs per SM leave the load latency
+// uncovered)
+template <class E> struct RsfAhead { static constexpr bool v = Emu<E>::v; };
 template <class E, int L>
 __host__ __device__ constexpr size_t rsf_smem() {
   return (size_t)(rc_twlen<E, L, rc_stages(L, RcLane<E>::P)>() +
-                  RsfShape<E, L>::NV * RsfShape<E, L>::Lx) *
+                  RsfShape<E, L>::NV * RsfShape<E, L>::Lx +
+                  (RsfAhead<E>::v ? RsfShape<E, L>::NV * L : 0)) *
              sizeof(E) +
          32 * sizeof(int);
 }
@@ -71,7 +76,12 @@ __global__ void __launch_bounds__(RsfShape<E, L>::T, (RsfOcc<E>::v))
   constexpr int TWN = rc_twlen<E, L, S>();
   E *stw = reinterpret_cast<E *>(fm_smem);
   E *xb = stw + TWN;
-  int *sexp = reinterpret_cast<int *>(xb + NV * Sh::Lx);
+  constexpr bool ahead = RsfAhead<E>::v;
+  // thread-private slots of the next batch's points
+  Raw *const slot =
+      reinterpret_cast<Raw *>(xb + NV * Sh::Lx) + threadIdx.x;
+  int *sexp =
+      reinterpret_cast<int *>(xb + NV * Sh::Lx + (ahead ? NV * L : 0));
   rc_fill_tw<E, L, 0>(stw, p.tw);
   __syncthreads();
   const int v = threadIdx.x % NV, t = threadIdx.x / NV;
@@ -79,15 +89,38 @@ __global__ void __launch_bounds__(RsfShape<E, L>::T, (RsfOcc<E>::v))
   const i64 Sx = p.es;
   const i64 nb = p.A * p.num_cols / NV;  // batches of NV adjacent vectors
   const FDiv dA((unsigned)p.A), dS((unsigned)Sx);
-  for (i64 bt = blockIdx.x; bt < nb; bt += gridDim.x) {
+  // column and row of point 0 of this thread's vector in batch bt
+  auto where = [&](i64 bt, unsigned &m) {
     const unsigned gv = (unsigned)(bt * NV);
-    const unsigned m = dA.div(gv), v0 = gv - m * (unsigned)p.A;
+    m = dA.div(gv);
+    const unsigned v0 = gv - m * (unsigned)p.A;
     const unsigned a = dS.div(v0), c0 = v0 - a * (unsigned)Sx;
-    const i64 row0 = (i64)a * L * Sx + c0 + v;
-    const Raw *src = (const Raw *)p.src + (i64)m * p.ld_src + row0;
+    return (i64)a * L * Sx + c0 + v;
+  };
+  auto prefetch = [&](i64 bt) {
+    unsigned m;
+    const i64 row0 = where(bt, m);
+    const Raw *q = (const Raw *)p.src + (i64)m * p.ld_src + row0 + (i64)t * Sx;
+#pragma unroll
+    for (int r = 0; r < P; ++r, q += G * Sx)
+      cp_async<sizeof(Raw)>(slot + Sh::T * r, q, true);
+    cp_async_commit();
+  };
+  if (ahead && blockIdx.x < nb) prefetch(blockIdx.x);
+  for (i64 bt = blockIdx.x; bt < nb; bt += gridDim.x) {
+    unsigned m;
+    const i64 row0 = where(bt, m);
     Raw d[P];
-    {
-      const Raw *q = src + (i64)t * Sx;
+    if constexpr (ahead) {
+      cp_async_wait<0>();
+      __syncwarp();
+#pragma unroll
+      for (int r = 0; r < P; ++r) d[r] = slot[Sh::T * r];
+      __syncwarp();
+      if (bt + gridDim.x < nb) prefetch(bt + gridDim.x);
+    } else {
+      const Raw *q = (const Raw *)p.src + (i64)m * p.ld_src + row0 +
+                     (i64)t * Sx;
 #pragma unroll
       for (int r = 0; r < P; ++r, q += G * Sx) d[r] = *q;
     }
