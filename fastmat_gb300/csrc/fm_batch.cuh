@@ -1,0 +1,298 @@
+// The batched persistent kernel (see the batch section of fm_vprog.cuh) and
+// the register transforms it runs on tiles.
+//
+// The passes of long transforms carry nearly all bytes of a batch (30.8 M of
+// 34.6 M element passes for 64 Circulant / Toeplitz / Fourier operators of
+// 64..65536 points).  As vector programs their tiles were bound by the
+// integer work of the generic loads and stores (about 45 % of the time) and
+// by the barriers between load, program and store; the register transforms
+// of fm_rfft.cuh load a tile's points into registers, transform and store
+// them directly, 8 points on each of the CTA's 512 threads.
+#pragma once
+
+#include "fm_rfft.cuh"
+
+namespace fmk {
+
+// Modes of a batch step's register transform
+enum {
+  RXM_NONE = 0,
+  RXM_FFT = 1,    // as rxfft_kernel, 64..512 points
+  RXM_CONV = 2    // as rxconv_kernel, 128..4096 points
+};
+constexpr int kRxbPoints = FM_MAX_THREADS * kRxP;  // points per tile
+// shared memory of a tile's exchange buffers
+constexpr size_t kRxbBytes = 38400;
+
+template <int L>
+__device__ __forceinline__ void rxb_fft(const RxStep &p, cfp<8> *xb,
+                                        unsigned tile) {
+  typedef cfp<8> E;
+  constexpr int P = kRxP, G = L / P, NV = kRxbPoints / L, T = FM_MAX_THREADS;
+  constexpr int S = rc_stages(L, P);
+  constexpr int R = rc_radix(S - 1, L, P);
+  constexpr int Lb = L + (L >> RcBuf<E, L>::SH);
+  constexpr int Lx = NV >= 16 ? (Lb | 1) : Lb + 16 / NV;
+  static_assert((size_t)NV * Lx * sizeof(E) <= kRxbBytes, "exchange buffers");
+  const int lane = threadIdx.x % NV, t = threadIdx.x / NV;
+  E *buf = xb + lane * Lx;
+  const unsigned nbc = (unsigned)((p.V + NV - 1) / NV);
+  const unsigned m = tile / nbc, v0 = (tile - m * nbc) * NV;
+  const unsigned v = v0 + lane;
+  const bool act = v < p.V;
+  const i64 col = (i64)m * p.ld_src;
+  float2 d[P];
+  if (p.in_cc == 1) {
+    // contiguous vectors: loads along their points, turned through the
+    // exchange buffer
+    float2 *rw = reinterpret_cast<float2 *>(xb);
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      const int k = threadIdx.x + T * i, vv = k / L, j = k % L;
+      const i64 row = (i64)(v0 + vv) * p.in_n + j;
+      float2 y = make_float2(0.f, 0.f);
+      if (v0 + vv < p.V && j < p.in_len && row < p.in_rows) {
+        const i64 srow = p.map_in ? p.map_in[row] : row;
+        if (srow >= 0) y = ((const float2 *)p.src)[col + srow];
+      }
+      rw[vv * Lx + rc_pad<E, L>(j)] = y;
+    }
+    __syncthreads();
+    const float2 *rr = rw + lane * Lx + rc_pad<E, L>(t);
+    const unsigned mask = p.conj_in ? 0x80000000u : 0u;
+#pragma unroll
+    for (int r = 0; r < P; ++r) d[r] = rx_conj(rr[rc_pad<E, L>(G * r)], mask);
+    __syncthreads();
+  }
+  const unsigned a = v / (unsigned)p.in_cc, c = v - a * (unsigned)p.in_cc;
+  const i64 rb = (i64)a * p.in_n * p.in_cc + c;
+  if (p.in_cc != 1) rx_load<E, L, true>(d, p, act, col, rb, t, G);
+  E x[P];
+#pragma unroll
+  for (int r = 0; r < P; ++r) x[r] = E{d[r].x, d[r].y};
+  rx_pre<E, L>(x, p, act, rb, t, G);
+  rc_forward<E, L, 0, -1, true, true>(x, buf, t, (const E *)p.tw);
+  if (act) {
+    const unsigned ao = v / (unsigned)p.out_cc,
+                   co = v - ao * (unsigned)p.out_cc;
+    rx_store<E, L, true>(x, 0, p, v, (i64)m * p.ld_dst,
+                   (i64)ao * p.out_n * p.out_cc + co,
+                   rc_nat<E, L>(rc_base<E, L, S - 1>(t)), [](int j) {
+                     return (j / R) * R + (j % R) * (L / R);
+                   });
+  }
+}
+
+template <int L>
+__device__ __forceinline__ void rxb_conv(const RxStep &p, cfp<8> *xb,
+                                           unsigned tile) {
+  typedef cfp<8> E;
+  constexpr int P = kRxP, G = L / P, VPC = kRxbPoints / L;
+  constexpr int S = rc_stages(L, P);
+  constexpr bool CTA = G > 32;
+  constexpr int Lc = RcBuf<E, L>::Lp;
+  static_assert((size_t)VPC * Lc * sizeof(E) <= kRxbBytes, "exchange buffers");
+  const int q = threadIdx.x / G, g = threadIdx.x % G;
+  E *buf = xb + q * Lc;
+  const unsigned gv = tile * VPC + q;
+  const bool act = gv < (unsigned)(p.V * p.num_cols);
+  const unsigned m = gv / (unsigned)p.V, v = gv - m * (unsigned)p.V;
+  const i64 rb = (i64)v * p.in_n;
+  float2 d[P];
+  rx_load<E, L, true>(d, p, act, (i64)m * p.ld_src, rb, g, G);
+  E x[P];
+#pragma unroll
+  for (int r = 0; r < P; ++r) x[r] = E{d[r].x, d[r].y};
+  rx_pre<E, L>(x, p, act, rb, g, G);
+  rc_forward<E, L, 0, -1, CTA, true>(x, buf, g, (const E *)p.tw);
+  if (act) {
+    const E *sp = (const E *)p.spec + (i64)v * p.spec_stride + g;
+#pragma unroll
+    for (int j = 0; j < P; ++j)
+      x[j] = mulv(x[j], tw_get<true>(sp, j * G), p.spec_conj != 0);
+  }
+  rc_inverse<E, L, S - 1, CTA, true>(x, buf, g, (const E *)p.tw);
+  if (act)
+    rx_store<E, L, true>(x, 0, p, v, (i64)m * p.ld_dst, (i64)v * p.out_n, g,
+                   [](int r) { return G * r; });
+}
+
+// one tile of a register step (complex64; called by all 512 threads, a
+// barrier follows)
+__device__ __forceinline__ void rx_batch_tile(const RxStep &p, int mode,
+                                           cfp<8> *xb, unsigned tile) {
+  switch (mode * 8192 + p.L) {
+    case RXM_FFT * 8192 + 64: rxb_fft<64>(p, xb, tile); break;
+    case RXM_FFT * 8192 + 128: rxb_fft<128>(p, xb, tile); break;
+    case RXM_FFT * 8192 + 256: rxb_fft<256>(p, xb, tile); break;
+    case RXM_FFT * 8192 + 512: rxb_fft<512>(p, xb, tile); break;
+    case RXM_CONV * 8192 + 128: rxb_conv<128>(p, xb, tile); break;
+    case RXM_CONV * 8192 + 256: rxb_conv<256>(p, xb, tile); break;
+    case RXM_CONV * 8192 + 512: rxb_conv<512>(p, xb, tile); break;
+    case RXM_CONV * 8192 + 1024: rxb_conv<1024>(p, xb, tile); break;
+    case RXM_CONV * 8192 + 2048: rxb_conv<2048>(p, xb, tile); break;
+    case RXM_CONV * 8192 + 4096: rxb_conv<4096>(p, xb, tile); break;
+    default: break;
+  }
+}
+
+// Loads of one batch tile into a slot: cp.async when the source already
+// has the compute type and needs no gather (completion is awaited later,
+// so the copy overlaps the previous tile's program), synchronous loads with
+// conversion and gather otherwise.
+// The launch record is first copied into shared memory (read there by
+// every op of the tile program instead of from global memory).
+template <class E>
+__device__ __forceinline__ void batch_issue_load(const Step *gp, Step *slot,
+                                                 E *sm, VInfo *vi, i64 tile,
+                                                 int tid, int T) {
+  {
+    static_assert(sizeof(Step) % 16 == 0, "launch record size");
+    const int4 *src = reinterpret_cast<const int4 *>(gp);
+    int4 *dst = reinterpret_cast<int4 *>(slot);
+    for (int i = tid; i < (int)(sizeof(Step) / 16); i += T) dst[i] = src[i];
+  }
+  __syncthreads();
+  const Step &p = *slot;
+  const i64 nvec = p.V * p.num_cols;
+  const FDiv dV((unsigned)p.V), dci((unsigned)p.vin.Cc),
+      dco((unsigned)p.vout.Cc);
+  setup_tile(p, vi, tile, dV, dci, dco, nvec, tid, T);
+  __syncthreads();
+  if (p.src_type == Tr<E>::code && !p.map_in)
+    load_async<E, 0>(p, sm, vi, tid, T);
+  else
+    load_general<E, 0>(p, sm, vi, tid, T);
+  cp_async_commit();
+}
+
+template <class E, int CLS>
+__global__ void __launch_bounds__(FM_MAX_THREADS, (MinBlocks<E, CLS>::v))
+    batch_kernel(const Step *__restrict__ steps, const i64 *__restrict__ start,
+                 const int *__restrict__ level, const RxStep *__restrict__ rx,
+                 const int *__restrict__ rxmode, int nlev, unsigned *bar,
+                 int *err, int max_B, size_t max_tile, long long wait_limit) {
+  extern __shared__ __align__(128) unsigned char fm_smem[];
+  const int tid = threadIdx.x, T = blockDim.x;
+  Step *const sst = reinterpret_cast<Step *>(fm_smem);
+  unsigned char *const h = fm_smem + batch_steps_bytes();
+  i64 *sq = reinterpret_cast<i64 *>(h);
+  // slot k: launch record, per-vector records, exponents and tile buffer
+  // (addresses recomputed on use to keep registers free)
+  const unsigned rec = (unsigned)((sizeof(VInfo) + 4) * max_B);
+  auto vis = [&](int k) {
+    return reinterpret_cast<VInfo *>(h + 8 * max_B + k * rec);
+  };
+  auto sexps = [&](int k) {
+    return reinterpret_cast<int *>(h + 8 * max_B + k * rec +
+                                   sizeof(VInfo) * max_B);
+  };
+  auto bufs = [&](int k) {
+    return reinterpret_cast<E *>(fm_smem + batch_head_bytes(max_B) +
+                                 k * max_tile);
+  };
+  const i64 G = gridDim.x;
+  // complex64: whether a step's tiles run as register transforms
+  auto mode = [&](int k) {
+    return std::is_same<E, float2>::value ? __ldg(rxmode + k) : 0;
+  };
+  __shared__ RxStep srx;  // record of the register step at hand
+  int rxk = -1;
+  for (int l = 0; l < nlev; ++l) {
+    const int s0 = level[l], s1 = level[l + 1];
+    const i64 t1 = start[s1];
+    // two-slot pipeline: the loads of tile g + G are issued before tile g
+    // is transformed and stored
+    i64 g = start[s0] + blockIdx.x;
+    int kc = s0, cur = 0;
+    if (g < t1) {
+      while (start[kc + 1] <= g) ++kc;
+      if (mode(kc) == 0)
+        batch_issue_load<E>(steps + kc, sst, bufs(0), vis(0), g - start[kc],
+                            tid, T);
+    }
+    for (; g < t1; g += G) {
+      const i64 gn = g + G;
+      int kn = kc;
+      if (gn < t1) {
+        while (start[kn + 1] <= gn) ++kn;
+        if (mode(kn) == 0)
+          batch_issue_load<E>(steps + kn, sst + (cur ^ 1), bufs(cur ^ 1),
+                              vis(cur ^ 1), gn - start[kn], tid, T);
+        else
+          cp_async_commit();  // (one group per tile)
+        cp_async_wait<1>();
+      } else {
+        cp_async_wait<0>();
+      }
+      if constexpr (std::is_same<E, float2>::value) {
+        const int md = mode(kc);
+        if (md != 0) {
+          // register transform: loads, transform and stores in one go, the
+          // tile buffer for its exchanges
+          if (rxk != kc) {
+            static_assert(sizeof(RxStep) % 8 == 0, "record size");
+            for (int i = tid; i < (int)(sizeof(RxStep) / 8); i += T)
+              reinterpret_cast<unsigned long long *>(&srx)[i] =
+                  reinterpret_cast<const unsigned long long *>(rx + kc)[i];
+            rxk = kc;
+          }
+          __syncthreads();
+          rx_batch_tile(srx, md, reinterpret_cast<cfp<8> *>(bufs(cur)),
+                        (unsigned)(g - start[kc]));
+          __syncthreads();
+          cur ^= 1;
+          kc = kn;
+          continue;
+        }
+      }
+      __syncthreads();
+      const Step &p = sst[cur];
+      E *sm = bufs(cur);
+      VInfo *vi = vis(cur);
+      int *sexp = sexps(cur);
+      const bool async = p.src_type == Tr<E>::code && !p.map_in;
+      if constexpr (Emu<E>::v) {
+        if (async) {
+          emu_in<E, 0>(p, sm, vi, sexp, tid, T);
+        } else {
+          for (int b = tid; b < p.B; b += T) sexp[b] = 0;
+        }
+        __syncthreads();
+      }
+      if (async && (p.conj_in || p.pre)) {
+        load_fixup<E, 0>(p, sm, vi, tid, T);
+        __syncthreads();
+      }
+      const int nwarps = T >> 5;
+      bool natural = false, stored = false;
+      if constexpr (std::is_same<E, float2>::value) {
+        if (p.rprog) {
+          // the program on registers; results in natural order (or already
+          // stored)
+          rt_program(p, sm, vi, tid, T);
+          natural = true;
+          stored = (p.rprog & RT_DIRECT) != 0;
+        }
+      }
+      if (natural) {
+      } else if (warp_mode<E, CLS, 0>(p.B, p.L, nwarps)) {
+        const int w = tid >> 5, vw = p.B / nwarps;
+        run_program<E, CLS, 0>(p, sm + w * vw * p.Lp, p.Lp, vw, vi + w * vw,
+                               sq + w * vw, tid & 31, 32);
+        __syncthreads();
+      } else {
+        run_program<E, CLS, 0>(p, sm, p.Lp, p.B, vi, sq, tid, T);
+      }
+      if (!stored) store_tile<E, 0>(p, sm, vi, sexp, tid, T, natural);
+      __syncthreads();
+      cur ^= 1;
+      kc = kn;
+    }
+    if (l + 1 < nlev &&
+        !grid_barrier(bar, (unsigned)(l + 1) * gridDim.x, err, wait_limit))
+      return;
+  }
+}
+
+}  // namespace fmk

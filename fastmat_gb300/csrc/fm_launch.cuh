@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include "fm_batch.cuh"
 #include "fm_rconv.cuh"
 #include "fm_rfft.cuh"
 #include "fm_rfwht.cuh"
@@ -35,6 +36,10 @@ struct BatchLaunch {
   const Step *steps = nullptr;  // device array, grouped by level
   const i64 *start = nullptr;   // first tile of every step (+ total)
   const int *level = nullptr;   // first step of every level (+ count)
+  // complex64: steps run as register transforms (fm_batch.cuh), their
+  // records and modes (0: vector program)
+  const RxStep *rx = nullptr;
+  const int *rxmode = nullptr;
   int nlev = 0;
   unsigned *bar = nullptr;      // grid-barrier counter, zero at launch
   int *err = nullptr;

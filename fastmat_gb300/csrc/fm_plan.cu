@@ -2526,6 +2526,54 @@ bool encode_view(CUtensorMap *tm, const void *base, const fmk::View &vw,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// the record of a register transform of long vectors for a bound launch
+fmk::RxStep rx_step(const LStep &ls, const fmk::Step &st) {
+  fmk::RxStep rx;
+  memset(&rx, 0, sizeof(rx));
+  rx.src = st.src;
+  rx.dst = st.dst;
+  rx.ld_src = st.ld_src;
+  rx.ld_dst = st.ld_dst;
+  rx.src_type = st.src_type;
+  rx.dst_type = st.dst_type;
+  rx.V = st.V;
+  rx.in_n = st.vin.n;
+  rx.in_cc = st.vin.Cc;
+  rx.out_n = st.vout.n;
+  rx.out_cc = st.vout.Cc;
+  rx.in_rows = st.in_rows;
+  rx.out_rows = st.out_rows;
+  rx.num_cols = st.num_cols;
+  rx.map_in = st.map_in;
+  rx.map_out = st.out_mode == 2 ? st.map_out : nullptr;
+  rx.pre = st.pre ? st.pre : ls.rc_pre;
+  rx.post = st.post ? st.post : ls.rc_post;
+  rx.pre_by_point = ls.rx_pre_pt;
+  rx.post_by_point = ls.rx_post_pt;
+  rx.spec = ls.rc_spec;
+  rx.spec_stride = ls.rx_spec_stride;
+  rx.tw = ls.rc_tw;
+  rx.wtab = ls.rx_w;
+  rx.wq = ls.rx_wq;
+  rx.wj = ls.rx_wj;
+  rx.in_len = st.in_len;
+  rx.out_len = st.out_len;
+  // an inverse FFT is the conjugate of the forward FFT of the conjugate
+  const int inv = ls.kind == 5 && ls.rc_sign > 0;
+  rx.conj_in = (st.conj_in || ls.rc_conj_in) != inv;
+  rx.conj_out = (st.conj_out || ls.rc_conj_out) != inv;
+  rx.pre_conj = inv;
+  rx.post_conj = inv;
+  rx.w_conj = (ls.rx_w_sign > 0) != inv;
+  rx.spec_conj = ls.rc_spec_conj;
+  rx.has_scale = st.has_scale;
+  rx.scale_re = st.scale_re;
+  rx.scale_im = inv ? -st.scale_im : st.scale_im;
+  rx.accumulate = st.accumulate;
+  rx.L = ls.rc_L;
+  return rx;
+}
+
 // Finish a bound launch (TMA descriptors, status word) and issue it.
 void launch_step(fm_plan *P, LStep &ls, fmk::Step &st, cudaStream_t s) {
   if (ls.pair == 2 && P->pair_done && !P->no_pair) {
@@ -2613,49 +2661,7 @@ void launch_step(fm_plan *P, LStep &ls, fmk::Step &st, cudaStream_t s) {
     // otherwise the equivalent vector program below
   }
   if (ls.kind == 5 || ls.kind == 6) {
-    fmk::RxStep rx;
-    memset(&rx, 0, sizeof(rx));
-    rx.src = st.src;
-    rx.dst = st.dst;
-    rx.ld_src = st.ld_src;
-    rx.ld_dst = st.ld_dst;
-    rx.src_type = st.src_type;
-    rx.dst_type = st.dst_type;
-    rx.V = st.V;
-    rx.in_n = st.vin.n;
-    rx.in_cc = st.vin.Cc;
-    rx.out_n = st.vout.n;
-    rx.out_cc = st.vout.Cc;
-    rx.in_rows = st.in_rows;
-    rx.out_rows = st.out_rows;
-    rx.num_cols = st.num_cols;
-    rx.map_in = st.map_in;
-    rx.map_out = st.out_mode == 2 ? st.map_out : nullptr;
-    rx.pre = st.pre ? st.pre : ls.rc_pre;
-    rx.post = st.post ? st.post : ls.rc_post;
-    rx.pre_by_point = ls.rx_pre_pt;
-    rx.post_by_point = ls.rx_post_pt;
-    rx.spec = ls.rc_spec;
-    rx.spec_stride = ls.rx_spec_stride;
-    rx.tw = ls.rc_tw;
-    rx.wtab = ls.rx_w;
-    rx.wq = ls.rx_wq;
-    rx.wj = ls.rx_wj;
-    rx.in_len = st.in_len;
-    rx.out_len = st.out_len;
-    // an inverse FFT is the conjugate of the forward FFT of the conjugate
-    const int inv = ls.kind == 5 && ls.rc_sign > 0;
-    rx.conj_in = (st.conj_in || ls.rc_conj_in) != inv;
-    rx.conj_out = (st.conj_out || ls.rc_conj_out) != inv;
-    rx.pre_conj = inv;
-    rx.post_conj = inv;
-    rx.w_conj = (ls.rx_w_sign > 0) != inv;
-    rx.spec_conj = ls.rc_spec_conj;
-    rx.has_scale = st.has_scale;
-    rx.scale_re = st.scale_re;
-    rx.scale_im = inv ? -st.scale_im : st.scale_im;
-    rx.accumulate = st.accumulate;
-    rx.L = ls.rc_L;
+    const fmk::RxStep rx = rx_step(ls, st);
     if (rx.V * rx.num_cols >= 0x7fffffffLL)
       fail(FM_ERR_UNSUPPORTED, "more than 2^31 vectors in one launch");
     const bool single = P->ctype == FM_C64;
@@ -3628,6 +3634,8 @@ int fm_batch_create(int32_t num_ops, fm_plan *const *plans,
       fmk::Step st;
       int cls;
       i64 tiles;
+      fmk::RxStep rx;  // register transform, when rxmode != 0
+      int rxmode;
     };
     std::vector<Item> items;
     std::vector<std::pair<int, size_t>> scratch_of;  // (op, bytes)
@@ -3724,12 +3732,28 @@ int fm_batch_create(int32_t num_ops, fm_plan *const *plans,
         st.err = B->status + 1;
         st.tma_in = st.tma_out = 0;
         st.rprog = ctype == FM_C64 ? rtile_shape(st) : 0;
-        const i64 tiles = (st.V * M + st.B - 1) / st.B;
+        i64 tiles = (st.V * M + st.B - 1) / st.B;
         if (st.V * M >= 0x7fffffffLL)
           fail(FM_ERR_UNSUPPORTED, "more than 2^31 vectors in one launch");
+        // passes of long transforms run as register transforms of 4096
+        // points per tile (fm_batch.cuh)
+        int rxmode = fmk::RXM_NONE;
+        fmk::RxStep rx;
+        memset(&rx, 0, sizeof(rx));
+        if (ctype == FM_C64 && st.src_type == FM_C64 &&
+            st.dst_type == FM_C64 && !st.accumulate && !st.has_scale &&
+            ((ls0.kind == 5 && ls0.rc_L >= 64 && ls0.rc_L <= 512) ||
+             (ls0.kind == 6 && ls0.rc_L >= 128))) {
+          rxmode = ls0.kind == 5 ? fmk::RXM_FFT : fmk::RXM_CONV;
+          rx = rx_step(ls0, st);
+          const i64 per = fmk::kRxbPoints / ls0.rc_L;
+          tiles = ls0.kind == 5 ? (st.V + per - 1) / per * M
+                                : (st.V * M + per - 1) / per;
+        }
         // the batch kernel has no class 5: its class 1 runs the same
         // program with the spectrum product as a separate op
-        items.push_back(Item{level++, st, ls.cls == 5 ? 1 : ls.cls, tiles});
+        items.push_back(Item{level++, st, ls.cls == 5 ? 1 : ls.cls, tiles,
+                             rx, rxmode});
       }
     }
     if (items.empty()) fail(FM_ERR_VALUE, "fm_batch_create: no work");
@@ -3738,14 +3762,18 @@ int fm_batch_create(int32_t num_ops, fm_plan *const *plans,
                        return a.level < b.level;
                      });
     // one kernel class that covers every program of the batch
-    int cls = items[0].cls;
+    int cls = -1;
     for (const Item &it : items) {
-      const int c = it.cls;
+      if (it.rxmode) continue;  // runs no vector program
+      const int c = cls < 0 ? cls = it.cls : it.cls;
       if (c == cls) continue;
       if (c == 0 || cls == 0 || c == 3 || cls == 3) cls = 0;
       else cls = 2;  // mixed power-of-two and odd-radix FFTs
     }
+    if (cls < 0) cls = 1;
     if (ctype == FM_C128_DF) cls = 0;
+    std::vector<fmk::RxStep> rxs;
+    std::vector<int> rxmodes;
     std::vector<fmk::Step> steps;
     std::vector<i64> start(1, 0);
     std::vector<int> level(1, 0);
@@ -3759,8 +3787,14 @@ int fm_batch_create(int32_t num_ops, fm_plan *const *plans,
         level_tiles = 0;
       }
       steps.push_back(items[k].st);
+      rxs.push_back(items[k].rx);
+      rxmodes.push_back(items[k].rxmode);
       start.push_back(start.back() + items[k].tiles);
       level_tiles += items[k].tiles;
+      if (items[k].rxmode) {
+        max_tile = std::max(max_tile, fmk::kRxbBytes);
+        continue;
+      }
       max_B = std::max(max_B, items[k].st.B);
       max_tile = std::max(max_tile, fmk::tile_bytes(items[k].st.B,
                                                    items[k].st.Lp, esz));
@@ -3788,6 +3822,20 @@ int fm_batch_create(int32_t num_ops, fm_plan *const *plans,
     CUDA_TRY(cudaMemcpy(dlevel, level.data(), level.size() * sizeof(int),
                         cudaMemcpyHostToDevice));
     fmk::BatchLaunch &L = B->launch;
+    if (ctype == FM_C64) {
+      fmk::RxStep *drx = nullptr;
+      int *dmode = nullptr;
+      CUDA_TRY(dev_malloc(&drx, rxs.size() * sizeof(fmk::RxStep)));
+      B->allocs.push_back(drx);
+      CUDA_TRY(dev_malloc(&dmode, rxmodes.size() * sizeof(int)));
+      B->allocs.push_back(dmode);
+      CUDA_TRY(cudaMemcpy(drx, rxs.data(), rxs.size() * sizeof(fmk::RxStep),
+                          cudaMemcpyHostToDevice));
+      CUDA_TRY(cudaMemcpy(dmode, rxmodes.data(), rxmodes.size() * sizeof(int),
+                          cudaMemcpyHostToDevice));
+      L.rx = drx;
+      L.rxmode = dmode;
+    }
     L.ctype = ctype;
     L.cls = cls;
     L.steps = dsteps;

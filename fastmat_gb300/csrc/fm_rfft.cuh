@@ -132,7 +132,8 @@ __device__ __forceinline__ float2 rx_zero(float2) {
 
 // P points j0 + dj r of one vector of the input view (row of point 0: rb,
 // column offset col) from any type, zero outside the vector or the column
-template <class E, int L>
+// (RAW: the buffer is known to hold the kernel's own type)
+template <class E, int L, bool RAW = false>
 __device__ __forceinline__ void rx_load(
     typename RxRaw<E>::type (&d)[RcLane<E>::P], const RxStep &p, bool act,
     i64 col, i64 rb, int j0, int dj) {
@@ -146,7 +147,12 @@ __device__ __forceinline__ void rx_load(
     Raw v = rx_zero(Raw());
     if (act && j < p.in_len && row < p.in_rows) {
       const i64 srow = p.map_in ? p.map_in[row] : row;
-      if (srow >= 0) v = load_as<Raw>(p.src, p.src_type, col + srow);
+      if (srow >= 0) {
+        if constexpr (RAW)
+          v = ((const Raw *)p.src)[col + srow];
+        else
+          v = load_as<Raw>(p.src, p.src_type, col + srow);
+      }
     }
     d[r] = v;
   }
@@ -214,7 +220,8 @@ __device__ __forceinline__ void rx_pre(E (&x)[RcLane<E>::P], const RxStep &p,
 }
 
 // registers to the output view: register r holds point j0 + jo(r)
-template <class E, int L, class JO>
+// (RAW: plain stores in the kernel's own type, no scalar)
+template <class E, int L, bool RAW = false, class JO>
 __device__ __forceinline__ void rx_store(E (&x)[RcLane<E>::P], int s,
                                          const RxStep &p, i64 v, i64 col,
                                          i64 rb, int j0, JO jo) {
@@ -239,12 +246,12 @@ __device__ __forceinline__ void rx_store(E (&x)[RcLane<E>::P], int s,
                     p.post_conj != 0);
     }
   }
-  if (p.has_scale) {
+  if (!RAW && p.has_scale) {
     const E c = scalar_of<E>(p.scale_re, p.scale_im);
 #pragma unroll
     for (int r = 0; r < P; ++r) x[r] = mulv(x[r], c, false);
   }
-  if (p.dst_type == Tr<E>::code && !p.accumulate) {
+  if (RAW || (p.dst_type == Tr<E>::code && !p.accumulate)) {
     const unsigned m = p.conj_out ? 0x80000000u : 0u;
     Raw *const dst = (Raw *)p.dst + col;
     if (p.map_out) {
@@ -271,15 +278,17 @@ __device__ __forceinline__ void rx_store(E (&x)[RcLane<E>::P], int s,
     }
     return;
   }
+  if constexpr (!RAW) {
 #pragma unroll
-  for (int r = 0; r < P; ++r) {
-    const int j = j0 + jo(r);
-    const i64 row = rb + (i64)j * cc;
-    if (j >= p.out_len || row >= p.out_rows) continue;
-    const i64 drow = p.map_out ? p.map_out[row] : row;
-    if (drow < 0) continue;
-    store_elem<E>(p.dst, p.dst_type, col + drow,
-                  p.conj_out ? conjv(x[r]) : x[r], p.accumulate != 0, s);
+    for (int r = 0; r < P; ++r) {
+      const int j = j0 + jo(r);
+      const i64 row = rb + (i64)j * cc;
+      if (j >= p.out_len || row >= p.out_rows) continue;
+      const i64 drow = p.map_out ? p.map_out[row] : row;
+      if (drow < 0) continue;
+      store_elem<E>(p.dst, p.dst_type, col + drow,
+                    p.conj_out ? conjv(x[r]) : x[r], p.accumulate != 0, s);
+    }
   }
 }
 

@@ -1965,132 +1965,4 @@ __host__ __device__ __forceinline__ size_t batch_smem(int max_B,
   return batch_head_bytes(max_B) + 2 * max_tile;
 }
 
-
-// Loads of one batch tile into a slot: cp.async when the source already
-// has the compute type and needs no gather (completion is awaited later,
-// so the copy overlaps the previous tile's program), synchronous loads with
-// conversion and gather otherwise.
-// The launch record is first copied into shared memory (read there by
-// every op of the tile program instead of from global memory).
-template <class E>
-__device__ __forceinline__ void batch_issue_load(const Step *gp, Step *slot,
-                                                 E *sm, VInfo *vi, i64 tile,
-                                                 int tid, int T) {
-  {
-    static_assert(sizeof(Step) % 16 == 0, "launch record size");
-    const int4 *src = reinterpret_cast<const int4 *>(gp);
-    int4 *dst = reinterpret_cast<int4 *>(slot);
-    for (int i = tid; i < (int)(sizeof(Step) / 16); i += T) dst[i] = src[i];
-  }
-  __syncthreads();
-  const Step &p = *slot;
-  const i64 nvec = p.V * p.num_cols;
-  const FDiv dV((unsigned)p.V), dci((unsigned)p.vin.Cc),
-      dco((unsigned)p.vout.Cc);
-  setup_tile(p, vi, tile, dV, dci, dco, nvec, tid, T);
-  __syncthreads();
-  if (p.src_type == Tr<E>::code && !p.map_in)
-    load_async<E, 0>(p, sm, vi, tid, T);
-  else
-    load_general<E, 0>(p, sm, vi, tid, T);
-  cp_async_commit();
-}
-
-template <class E, int CLS>
-__global__ void __launch_bounds__(FM_MAX_THREADS, (MinBlocks<E, CLS>::v))
-    batch_kernel(const Step *__restrict__ steps, const i64 *__restrict__ start,
-                 const int *__restrict__ level, int nlev, unsigned *bar,
-                 int *err, int max_B, size_t max_tile, long long wait_limit) {
-  extern __shared__ __align__(128) unsigned char fm_smem[];
-  const int tid = threadIdx.x, T = blockDim.x;
-  Step *const sst = reinterpret_cast<Step *>(fm_smem);
-  unsigned char *const h = fm_smem + batch_steps_bytes();
-  i64 *sq = reinterpret_cast<i64 *>(h);
-  // slot k: launch record, per-vector records, exponents and tile buffer
-  // (addresses recomputed on use to keep registers free)
-  const unsigned rec = (unsigned)((sizeof(VInfo) + 4) * max_B);
-  auto vis = [&](int k) {
-    return reinterpret_cast<VInfo *>(h + 8 * max_B + k * rec);
-  };
-  auto sexps = [&](int k) {
-    return reinterpret_cast<int *>(h + 8 * max_B + k * rec +
-                                   sizeof(VInfo) * max_B);
-  };
-  auto bufs = [&](int k) {
-    return reinterpret_cast<E *>(fm_smem + batch_head_bytes(max_B) +
-                                 k * max_tile);
-  };
-  const i64 G = gridDim.x;
-  for (int l = 0; l < nlev; ++l) {
-    const int s0 = level[l], s1 = level[l + 1];
-    const i64 t1 = start[s1];
-    // two-slot pipeline: the loads of tile g + G are issued before tile g
-    // is transformed and stored
-    i64 g = start[s0] + blockIdx.x;
-    int kc = s0, cur = 0;
-    if (g < t1) {
-      while (start[kc + 1] <= g) ++kc;
-      batch_issue_load<E>(steps + kc, sst, bufs(0), vis(0), g - start[kc],
-                          tid, T);
-    }
-    for (; g < t1; g += G) {
-      const i64 gn = g + G;
-      int kn = kc;
-      if (gn < t1) {
-        while (start[kn + 1] <= gn) ++kn;
-        batch_issue_load<E>(steps + kn, sst + (cur ^ 1), bufs(cur ^ 1),
-                            vis(cur ^ 1), gn - start[kn], tid, T);
-        cp_async_wait<1>();
-      } else {
-        cp_async_wait<0>();
-      }
-      __syncthreads();
-      const Step &p = sst[cur];
-      E *sm = bufs(cur);
-      VInfo *vi = vis(cur);
-      int *sexp = sexps(cur);
-      const bool async = p.src_type == Tr<E>::code && !p.map_in;
-      if constexpr (Emu<E>::v) {
-        if (async) {
-          emu_in<E, 0>(p, sm, vi, sexp, tid, T);
-        } else {
-          for (int b = tid; b < p.B; b += T) sexp[b] = 0;
-        }
-        __syncthreads();
-      }
-      if (async && (p.conj_in || p.pre)) {
-        load_fixup<E, 0>(p, sm, vi, tid, T);
-        __syncthreads();
-      }
-      const int nwarps = T >> 5;
-      bool natural = false, stored = false;
-      if constexpr (std::is_same<E, float2>::value) {
-        if (p.rprog) {
-          // the program on registers; results in natural order (or already
-          // stored)
-          rt_program(p, sm, vi, tid, T);
-          natural = true;
-          stored = (p.rprog & RT_DIRECT) != 0;
-        }
-      }
-      if (natural) {
-      } else if (warp_mode<E, CLS, 0>(p.B, p.L, nwarps)) {
-        const int w = tid >> 5, vw = p.B / nwarps;
-        run_program<E, CLS, 0>(p, sm + w * vw * p.Lp, p.Lp, vw, vi + w * vw,
-                               sq + w * vw, tid & 31, 32);
-        __syncthreads();
-      } else {
-        run_program<E, CLS, 0>(p, sm, p.Lp, p.B, vi, sq, tid, T);
-      }
-      if (!stored) store_tile<E, 0>(p, sm, vi, sexp, tid, T, natural);
-      __syncthreads();
-      cur ^= 1;
-      kc = kn;
-    }
-    if (l + 1 < nlev &&
-        !grid_barrier(bar, (unsigned)(l + 1) * gridDim.x, err, wait_limit))
-      return;
-  }
-}
-
 }  // namespace fmk
