@@ -6,8 +6,9 @@
 // 64..65536 points).  As vector programs their tiles were bound by the
 // integer work of the generic loads and stores (about 45 % of the time) and
 // by the barriers between load, program and store; the register transforms
-// of fm_rfft.cuh load a tile's points into registers, transform and store
-// them directly, 8 points on each of the CTA's 512 threads.
+// of fm_rfft.cuh take a tile's points, copied ahead, into registers,
+// transform and store them directly, 8 points on each of the CTA's 512
+// threads.
 #pragma once
 
 #include "fm_rfft.cuh"
@@ -24,6 +25,68 @@ constexpr int kRxbPoints = FM_MAX_THREADS * kRxP;  // points per tile
 // shared memory of a tile's exchange buffers
 constexpr size_t kRxbBytes = 38400;
 
+// exchange buffer stride of rxb_fft's vectors (the rule of RxShape::Lx)
+__host__ __device__ constexpr int rxb_lx(int L) {
+  return kRxbPoints / L >= 16 ? ((L + (L >> 3)) | 1)
+                              : L + (L >> 3) + 16 / (kRxbPoints / L);
+}
+
+// Copy a tile's points ahead into its buffer (cp.async, zeros where there
+// are none): the points of thread k at k + 512 r, or, for contiguous vectors
+// that rxb_fft turns, along the vectors at their padded positions.
+__device__ __forceinline__ void rxb_issue(const RxStep &p, int mode,
+                                          float2 *slot, unsigned tile) {
+  constexpr int T = FM_MAX_THREADS;
+  const int L = p.L, G = L / kRxP, NV = kRxbPoints / L;
+  const int tid = threadIdx.x;
+  unsigned m, v;
+  int j0;
+  if (mode == RXM_FFT) {
+    const unsigned nbc = ((unsigned)p.V + NV - 1) / NV;
+    m = tile / nbc;
+    v = (tile - m * nbc) * NV;  // first vector
+    if (p.in_cc == 1) {
+      const int lg = __ffs(L) - 1, Lx = rxb_lx(L);
+      const i64 col = (i64)m * p.ld_src;
+#pragma unroll
+      for (int i = 0; i < kRxP; ++i) {
+        const int k = tid + T * i, vv = k >> lg, j = k & (L - 1);
+        const i64 row = (i64)(v + vv) * p.in_n + j;
+        i64 at = v + vv < p.V && j < p.in_len && row < p.in_rows ? row : -1;
+        if (p.map_in && at >= 0) at = p.map_in[at];
+        cp_async<8>(slot + vv * Lx + j + (j >> 3),
+                    at >= 0 ? (const void *)((const float2 *)p.src + col + at)
+                            : p.src,
+                    at >= 0);
+      }
+      return;
+    }
+    v += tid & (NV - 1);
+    j0 = tid / NV;
+  } else {
+    const unsigned gv = tile * NV + tid / G;
+    m = gv / (unsigned)p.V;
+    v = gv - m * (unsigned)p.V;
+    if (gv >= (unsigned)(p.V * p.num_cols)) v = (unsigned)p.V;  // none
+    j0 = tid & (G - 1);
+  }
+  const i64 cc = p.in_cc;
+  const unsigned a = v / (unsigned)cc, c = v - a * (unsigned)cc;
+  const i64 rb = (i64)a * p.in_n * cc + c;
+  const i64 col = (i64)m * p.ld_src;
+#pragma unroll
+  for (int r = 0; r < kRxP; ++r) {
+    const int j = j0 + G * r;
+    const i64 row = rb + (i64)j * cc;
+    i64 at = v < p.V && j < p.in_len && row < p.in_rows ? row : -1;
+    if (p.map_in && at >= 0) at = p.map_in[at];
+    cp_async<8>(slot + tid + T * r,
+                at >= 0 ? (const void *)((const float2 *)p.src + col + at)
+                        : p.src,
+                at >= 0);
+  }
+}
+
 template <int L>
 __device__ __forceinline__ void rxb_fft(const RxStep &p, cfp<8> *xb,
                                         unsigned tile) {
@@ -31,63 +94,54 @@ __device__ __forceinline__ void rxb_fft(const RxStep &p, cfp<8> *xb,
   constexpr int P = kRxP, G = L / P, NV = kRxbPoints / L, T = FM_MAX_THREADS;
   constexpr int S = rc_stages(L, P);
   constexpr int R = rc_radix(S - 1, L, P);
-  constexpr int Lb = L + (L >> RcBuf<E, L>::SH);
-  constexpr int Lx = NV >= 16 ? (Lb | 1) : Lb + 16 / NV;
+  constexpr int Lx = rxb_lx(L);
+  static_assert(RcBuf<E, L>::SH == 3, "padding of rxb_issue");
   static_assert((size_t)NV * Lx * sizeof(E) <= kRxbBytes, "exchange buffers");
   const int lane = threadIdx.x % NV, t = threadIdx.x / NV;
   E *buf = xb + lane * Lx;
   const unsigned nbc = (unsigned)((p.V + NV - 1) / NV);
-  const unsigned m = tile / nbc, v0 = (tile - m * nbc) * NV;
-  const unsigned v = v0 + lane;
+  const unsigned m = tile / nbc, v = (tile - m * nbc) * NV + lane;
   const bool act = v < p.V;
-  const i64 col = (i64)m * p.ld_src;
-  float2 d[P];
-  if (p.in_cc == 1) {
-    // contiguous vectors: loads along their points, turned through the
-    // exchange buffer
-    float2 *rw = reinterpret_cast<float2 *>(xb);
-#pragma unroll
-    for (int i = 0; i < P; ++i) {
-      const int k = threadIdx.x + T * i, vv = k / L, j = k % L;
-      const i64 row = (i64)(v0 + vv) * p.in_n + j;
-      float2 y = make_float2(0.f, 0.f);
-      if (v0 + vv < p.V && j < p.in_len && row < p.in_rows) {
-        const i64 srow = p.map_in ? p.map_in[row] : row;
-        if (srow >= 0) y = ((const float2 *)p.src)[col + srow];
-      }
-      rw[vv * Lx + rc_pad<E, L>(j)] = y;
-    }
-    __syncthreads();
-    const float2 *rr = rw + lane * Lx + rc_pad<E, L>(t);
-    const unsigned mask = p.conj_in ? 0x80000000u : 0u;
-#pragma unroll
-    for (int r = 0; r < P; ++r) d[r] = rx_conj(rr[rc_pad<E, L>(G * r)], mask);
-    __syncthreads();
-  }
-  const unsigned a = v / (unsigned)p.in_cc, c = v - a * (unsigned)p.in_cc;
-  const i64 rb = (i64)a * p.in_n * p.in_cc + c;
-  if (p.in_cc != 1) rx_load<E, L, true>(d, p, act, col, rb, t, G);
+  const unsigned mask = p.conj_in ? 0x80000000u : 0u;
+  const float2 *raw = reinterpret_cast<const float2 *>(xb);
   E x[P];
+  if (p.in_cc == 1) {
+    const float2 *rr = raw + lane * Lx + rc_pad<E, L>(t);
 #pragma unroll
-  for (int r = 0; r < P; ++r) x[r] = E{d[r].x, d[r].y};
-  rx_pre<E, L>(x, p, act, rb, t, G);
+    for (int r = 0; r < P; ++r) {
+      const float2 d = rx_conj(rr[rc_pad<E, L>(G * r)], mask);
+      x[r] = E{d.x, d.y};
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < P; ++r) {
+      const float2 d = rx_conj(raw[threadIdx.x + T * r], mask);
+      x[r] = E{d.x, d.y};
+    }
+  }
+  __syncthreads();  // the exchanges reuse the buffer
+  if (p.pre) {
+    const unsigned a = v / (unsigned)p.in_cc, c = v - a * (unsigned)p.in_cc;
+    rx_pre<E, L>(x, p, act, (i64)a * p.in_n * p.in_cc + c, t, G);
+  }
   rc_forward<E, L, 0, -1, true, true>(x, buf, t, (const E *)p.tw);
   if (act) {
     const unsigned ao = v / (unsigned)p.out_cc,
                    co = v - ao * (unsigned)p.out_cc;
     rx_store<E, L, true>(x, 0, p, v, (i64)m * p.ld_dst,
-                   (i64)ao * p.out_n * p.out_cc + co,
-                   rc_nat<E, L>(rc_base<E, L, S - 1>(t)), [](int j) {
-                     return (j / R) * R + (j % R) * (L / R);
-                   });
+                         (i64)ao * p.out_n * p.out_cc + co,
+                         rc_nat<E, L>(rc_base<E, L, S - 1>(t)), [](int j) {
+                           return (j / R) * R + (j % R) * (L / R);
+                         });
   }
 }
 
 template <int L>
 __device__ __forceinline__ void rxb_conv(const RxStep &p, cfp<8> *xb,
-                                           unsigned tile) {
+                                         unsigned tile) {
   typedef cfp<8> E;
-  constexpr int P = kRxP, G = L / P, VPC = kRxbPoints / L;
+  constexpr int P = kRxP, G = L / P, VPC = kRxbPoints / L,
+                T = FM_MAX_THREADS;
   constexpr int S = rc_stages(L, P);
   constexpr bool CTA = G > 32;
   constexpr int Lc = RcBuf<E, L>::Lp;
@@ -97,13 +151,16 @@ __device__ __forceinline__ void rxb_conv(const RxStep &p, cfp<8> *xb,
   const unsigned gv = tile * VPC + q;
   const bool act = gv < (unsigned)(p.V * p.num_cols);
   const unsigned m = gv / (unsigned)p.V, v = gv - m * (unsigned)p.V;
-  const i64 rb = (i64)v * p.in_n;
-  float2 d[P];
-  rx_load<E, L, true>(d, p, act, (i64)m * p.ld_src, rb, g, G);
+  const unsigned mask = p.conj_in ? 0x80000000u : 0u;
+  const float2 *raw = reinterpret_cast<const float2 *>(xb);
   E x[P];
 #pragma unroll
-  for (int r = 0; r < P; ++r) x[r] = E{d[r].x, d[r].y};
-  rx_pre<E, L>(x, p, act, rb, g, G);
+  for (int r = 0; r < P; ++r) {
+    const float2 d = rx_conj(raw[threadIdx.x + T * r], mask);
+    x[r] = E{d.x, d.y};
+  }
+  __syncthreads();  // the exchanges reuse the buffer
+  rx_pre<E, L>(x, p, act, (i64)v * p.in_n, g, G);
   rc_forward<E, L, 0, -1, CTA, true>(x, buf, g, (const E *)p.tw);
   if (act) {
     const E *sp = (const E *)p.spec + (i64)v * p.spec_stride + g;
@@ -114,7 +171,7 @@ __device__ __forceinline__ void rxb_conv(const RxStep &p, cfp<8> *xb,
   rc_inverse<E, L, S - 1, CTA, true>(x, buf, g, (const E *)p.tw);
   if (act)
     rx_store<E, L, true>(x, 0, p, v, (i64)m * p.ld_dst, (i64)v * p.out_n, g,
-                   [](int r) { return G * r; });
+                         [](int r) { return G * r; });
 }
 
 // one tile of a register step (complex64; called by all 512 threads, a
@@ -196,8 +253,29 @@ __global__ void __launch_bounds__(FM_MAX_THREADS, (MinBlocks<E, CLS>::v))
   auto mode = [&](int k) {
     return std::is_same<E, float2>::value ? __ldg(rxmode + k) : 0;
   };
-  __shared__ RxStep srx;  // record of the register step at hand
-  int rxk = -1;
+  // records of the register steps in the two slots, and which steps
+  __shared__ RxStep srx[2];
+  int rxk[2] = {-1, -1};
+  // loads of tile `at` of step k into slot c (one cp.async group)
+  auto issue = [&](int k, int c, i64 at) {
+    const int md = mode(k);
+    if (md == 0) {
+      batch_issue_load<E>(steps + k, sst + c, bufs(c), vis(c), at, tid, T);
+      return;
+    }
+    if constexpr (std::is_same<E, float2>::value) {
+      if (rxk[c] != k) {
+        static_assert(sizeof(RxStep) % 8 == 0, "record size");
+        for (int i = tid; i < (int)(sizeof(RxStep) / 8); i += T)
+          reinterpret_cast<unsigned long long *>(srx + c)[i] =
+              reinterpret_cast<const unsigned long long *>(rx + k)[i];
+        rxk[c] = k;
+        __syncthreads();
+      }
+      rxb_issue(srx[c], md, bufs(c), (unsigned)at);
+      cp_async_commit();
+    }
+  };
   for (int l = 0; l < nlev; ++l) {
     const int s0 = level[l], s1 = level[l + 1];
     const i64 t1 = start[s1];
@@ -207,20 +285,14 @@ __global__ void __launch_bounds__(FM_MAX_THREADS, (MinBlocks<E, CLS>::v))
     int kc = s0, cur = 0;
     if (g < t1) {
       while (start[kc + 1] <= g) ++kc;
-      if (mode(kc) == 0)
-        batch_issue_load<E>(steps + kc, sst, bufs(0), vis(0), g - start[kc],
-                            tid, T);
+      issue(kc, 0, g - start[kc]);
     }
     for (; g < t1; g += G) {
       const i64 gn = g + G;
       int kn = kc;
       if (gn < t1) {
         while (start[kn + 1] <= gn) ++kn;
-        if (mode(kn) == 0)
-          batch_issue_load<E>(steps + kn, sst + (cur ^ 1), bufs(cur ^ 1),
-                              vis(cur ^ 1), gn - start[kn], tid, T);
-        else
-          cp_async_commit();  // (one group per tile)
+        issue(kn, cur ^ 1, gn - start[kn]);
         cp_async_wait<1>();
       } else {
         cp_async_wait<0>();
@@ -228,17 +300,8 @@ __global__ void __launch_bounds__(FM_MAX_THREADS, (MinBlocks<E, CLS>::v))
       if constexpr (std::is_same<E, float2>::value) {
         const int md = mode(kc);
         if (md != 0) {
-          // register transform: loads, transform and stores in one go, the
-          // tile buffer for its exchanges
-          if (rxk != kc) {
-            static_assert(sizeof(RxStep) % 8 == 0, "record size");
-            for (int i = tid; i < (int)(sizeof(RxStep) / 8); i += T)
-              reinterpret_cast<unsigned long long *>(&srx)[i] =
-                  reinterpret_cast<const unsigned long long *>(rx + kc)[i];
-            rxk = kc;
-          }
           __syncthreads();
-          rx_batch_tile(srx, md, reinterpret_cast<cfp<8> *>(bufs(cur)),
+          rx_batch_tile(srx[cur], md, reinterpret_cast<cfp<8> *>(bufs(cur)),
                         (unsigned)(g - start[kc]));
           __syncthreads();
           cur ^= 1;
