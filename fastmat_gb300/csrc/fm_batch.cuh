@@ -25,32 +25,50 @@ constexpr int kRxbPoints = FM_MAX_THREADS * kRxP;  // points per tile
 // shared memory of a tile's exchange buffers
 constexpr size_t kRxbBytes = 38400;
 
-// exchange buffer stride of rxb_fft's vectors (the rule of RxShape::Lx)
+// rxb_fft works in groups of threads with barriers of their own: 256
+// threads up to 256 points (rows of 64 bytes or more), all 512 above
+__host__ __device__ constexpr int rxb_group(int L) {
+  return L <= 256 ? 256 : FM_MAX_THREADS;
+}
+// adjacent vectors of a group, and the stride of their exchange buffers
+// (the rule of RxShape::Lx)
+__host__ __device__ constexpr int rxb_nv(int L) {
+  return rxb_group(L) * kRxP / L;
+}
 __host__ __device__ constexpr int rxb_lx(int L) {
-  return kRxbPoints / L >= 16 ? ((L + (L >> 3)) | 1)
-                              : L + (L >> 3) + 16 / (kRxbPoints / L);
+  return rxb_nv(L) >= 16 ? ((L + (L >> 3)) | 1)
+                         : L + (L >> 3) + 16 / rxb_nv(L);
+}
+// words between the groups' buffers
+__host__ __device__ constexpr int rxb_region(int L) {
+  return rxb_nv(L) * rxb_lx(L);
 }
 
 // Copy a tile's points ahead into its buffer (cp.async, zeros where there
-// are none): the points of thread k at k + 512 r, or, for contiguous vectors
-// that rxb_fft turns, along the vectors at their padded positions.
+// are none).  FFT: the points of thread k of a group at k + T r of the
+// group's region, or, for contiguous vectors that rxb_fft turns, along the
+// vectors at their padded positions; convolution: point j of a vector at j of
+// its exchange buffer.
 __device__ __forceinline__ void rxb_issue(const RxStep &p, int mode,
                                           float2 *slot, unsigned tile) {
-  constexpr int T = FM_MAX_THREADS;
-  const int L = p.L, G = L / kRxP, NV = kRxbPoints / L;
+  const int L = p.L, G = L / kRxP;
   const int tid = threadIdx.x;
   unsigned m, v;
-  int j0;
+  int j0, step;
   if (mode == RXM_FFT) {
+    const int T = rxb_group(L), NV = rxb_nv(L), grp = tid / T, k0 = tid % T;
     const unsigned nbc = ((unsigned)p.V + NV - 1) / NV;
-    m = tile / nbc;
-    v = (tile - m * nbc) * NV;  // first vector
+    const unsigned bt = tile * (FM_MAX_THREADS / T) + grp;
+    m = bt / nbc;
+    v = (bt - m * nbc) * NV;  // first vector
+    if (m >= (unsigned)p.num_cols) v = (unsigned)p.V;  // none
+    slot += grp * rxb_region(L);
     if (p.in_cc == 1) {
       const int lg = __ffs(L) - 1, Lx = rxb_lx(L);
       const i64 col = (i64)m * p.ld_src;
 #pragma unroll
       for (int i = 0; i < kRxP; ++i) {
-        const int k = tid + T * i, vv = k >> lg, j = k & (L - 1);
+        const int k = k0 + T * i, vv = k >> lg, j = k & (L - 1);
         const i64 row = (i64)(v + vv) * p.in_n + j;
         i64 at = v + vv < p.V && j < p.in_len && row < p.in_rows ? row : -1;
         if (p.map_in && at >= 0) at = p.map_in[at];
@@ -61,29 +79,41 @@ __device__ __forceinline__ void rxb_issue(const RxStep &p, int mode,
       }
       return;
     }
-    v += tid & (NV - 1);
-    j0 = tid / NV;
+    v += k0 & (NV - 1);
+    j0 = k0 / NV;
+    slot += k0;
+    step = T;
   } else {
-    const unsigned gv = tile * NV + tid / G;
+    const int q = tid / G;
+    const unsigned gv = tile * (kRxbPoints / L) + q;
     m = gv / (unsigned)p.V;
     v = gv - m * (unsigned)p.V;
     if (gv >= (unsigned)(p.V * p.num_cols)) v = (unsigned)p.V;  // none
     j0 = tid & (G - 1);
+    slot += q * (L + (L >> 3)) + j0;
+    step = G;
   }
   const i64 cc = p.in_cc;
   const unsigned a = v / (unsigned)cc, c = v - a * (unsigned)cc;
   const i64 rb = (i64)a * p.in_n * cc + c;
-  const i64 col = (i64)m * p.ld_src;
+  const float2 *src = (const float2 *)p.src + (i64)m * p.ld_src;
+  if (v < p.V && !p.map_in && p.in_len == L &&
+      rb + (i64)(L - 1) * cc < p.in_rows) {
+    const float2 *s = src + rb + (i64)j0 * cc;
+    const i64 d = (i64)G * cc;
 #pragma unroll
-  for (int r = 0; r < kRxP; ++r) {
-    const int j = j0 + G * r;
-    const i64 row = rb + (i64)j * cc;
-    i64 at = v < p.V && j < p.in_len && row < p.in_rows ? row : -1;
-    if (p.map_in && at >= 0) at = p.map_in[at];
-    cp_async<8>(slot + tid + T * r,
-                at >= 0 ? (const void *)((const float2 *)p.src + col + at)
-                        : p.src,
-                at >= 0);
+    for (int r = 0; r < kRxP; ++r, s += d)
+      cp_async<8>(slot + step * r, s, true);
+  } else {
+#pragma unroll
+    for (int r = 0; r < kRxP; ++r) {
+      const int j = j0 + G * r;
+      const i64 row = rb + (i64)j * cc;
+      i64 at = v < p.V && j < p.in_len && row < p.in_rows ? row : -1;
+      if (p.map_in && at >= 0) at = p.map_in[at];
+      cp_async<8>(slot + step * r,
+                  at >= 0 ? (const void *)(src + at) : p.src, at >= 0);
+    }
   }
 }
 
@@ -91,17 +121,23 @@ template <int L>
 __device__ __forceinline__ void rxb_fft(const RxStep &p, cfp<8> *xb,
                                         unsigned tile) {
   typedef cfp<8> E;
-  constexpr int P = kRxP, G = L / P, NV = kRxbPoints / L, T = FM_MAX_THREADS;
+  constexpr int P = kRxP, G = L / P, T = rxb_group(L), NV = rxb_nv(L);
+  constexpr int SY = T == FM_MAX_THREADS ? 1 : T;
   constexpr int S = rc_stages(L, P);
   constexpr int R = rc_radix(S - 1, L, P);
   constexpr int Lx = rxb_lx(L);
   static_assert(RcBuf<E, L>::SH == 3, "padding of rxb_issue");
-  static_assert((size_t)NV * Lx * sizeof(E) <= kRxbBytes, "exchange buffers");
-  const int lane = threadIdx.x % NV, t = threadIdx.x / NV;
+  static_assert((size_t)FM_MAX_THREADS / T * rxb_region(L) * sizeof(E) <=
+                    kRxbBytes,
+                "exchange buffers");
+  const int grp = threadIdx.x / T, k0 = threadIdx.x % T;
+  const int lane = k0 % NV, t = k0 / NV;
+  xb += grp * rxb_region(L);
   E *buf = xb + lane * Lx;
   const unsigned nbc = (unsigned)((p.V + NV - 1) / NV);
-  const unsigned m = tile / nbc, v = (tile - m * nbc) * NV + lane;
-  const bool act = v < p.V;
+  const unsigned bt = tile * (FM_MAX_THREADS / T) + grp;
+  const unsigned m = bt / nbc, v = (bt - m * nbc) * NV + lane;
+  const bool act = v < p.V && m < p.num_cols;
   const unsigned mask = p.conj_in ? 0x80000000u : 0u;
   const float2 *raw = reinterpret_cast<const float2 *>(xb);
   E x[P];
@@ -115,16 +151,16 @@ __device__ __forceinline__ void rxb_fft(const RxStep &p, cfp<8> *xb,
   } else {
 #pragma unroll
     for (int r = 0; r < P; ++r) {
-      const float2 d = rx_conj(raw[threadIdx.x + T * r], mask);
+      const float2 d = rx_conj(raw[k0 + T * r], mask);
       x[r] = E{d.x, d.y};
     }
   }
-  __syncthreads();  // the exchanges reuse the buffer
+  rc_sync<SY>();  // the exchanges reuse the buffer
   if (p.pre) {
     const unsigned a = v / (unsigned)p.in_cc, c = v - a * (unsigned)p.in_cc;
     rx_pre<E, L>(x, p, act, (i64)a * p.in_n * p.in_cc + c, t, G);
   }
-  rc_forward<E, L, 0, -1, true, true>(x, buf, t, (const E *)p.tw);
+  rc_forward<E, L, 0, -1, SY, true>(x, buf, t, (const E *)p.tw);
   if (act) {
     const unsigned ao = v / (unsigned)p.out_cc,
                    co = v - ao * (unsigned)p.out_cc;
@@ -140,11 +176,12 @@ template <int L>
 __device__ __forceinline__ void rxb_conv(const RxStep &p, cfp<8> *xb,
                                          unsigned tile) {
   typedef cfp<8> E;
-  constexpr int P = kRxP, G = L / P, VPC = kRxbPoints / L,
-                T = FM_MAX_THREADS;
+  constexpr int P = kRxP, G = L / P, VPC = kRxbPoints / L;
+  // the threads of one vector: a warp or less, a group, the CTA
+  constexpr int SY = G <= 32 ? 0 : G == FM_MAX_THREADS ? 1 : G;
   constexpr int S = rc_stages(L, P);
-  constexpr bool CTA = G > 32;
   constexpr int Lc = RcBuf<E, L>::Lp;
+  static_assert(Lc == L + (L >> 3), "buffers of rxb_issue");
   static_assert((size_t)VPC * Lc * sizeof(E) <= kRxbBytes, "exchange buffers");
   const int q = threadIdx.x / G, g = threadIdx.x % G;
   E *buf = xb + q * Lc;
@@ -152,23 +189,23 @@ __device__ __forceinline__ void rxb_conv(const RxStep &p, cfp<8> *xb,
   const bool act = gv < (unsigned)(p.V * p.num_cols);
   const unsigned m = gv / (unsigned)p.V, v = gv - m * (unsigned)p.V;
   const unsigned mask = p.conj_in ? 0x80000000u : 0u;
-  const float2 *raw = reinterpret_cast<const float2 *>(xb);
+  const float2 *raw = reinterpret_cast<const float2 *>(buf) + g;
   E x[P];
 #pragma unroll
   for (int r = 0; r < P; ++r) {
-    const float2 d = rx_conj(raw[threadIdx.x + T * r], mask);
+    const float2 d = rx_conj(raw[G * r], mask);
     x[r] = E{d.x, d.y};
   }
-  __syncthreads();  // the exchanges reuse the buffer
+  rc_sync<SY>();  // the exchanges reuse the buffer
   rx_pre<E, L>(x, p, act, (i64)v * p.in_n, g, G);
-  rc_forward<E, L, 0, -1, CTA, true>(x, buf, g, (const E *)p.tw);
+  rc_forward<E, L, 0, -1, SY, true>(x, buf, g, (const E *)p.tw);
   if (act) {
     const E *sp = (const E *)p.spec + (i64)v * p.spec_stride + g;
 #pragma unroll
     for (int j = 0; j < P; ++j)
       x[j] = mulv(x[j], tw_get<true>(sp, j * G), p.spec_conj != 0);
   }
-  rc_inverse<E, L, S - 1, CTA, true>(x, buf, g, (const E *)p.tw);
+  rc_inverse<E, L, S - 1, SY, true>(x, buf, g, (const E *)p.tw);
   if (act)
     rx_store<E, L, true>(x, 0, p, v, (i64)m * p.ld_dst, (i64)v * p.out_n, g,
                          [](int r) { return G * r; });

@@ -3746,9 +3746,17 @@ int fm_batch_create(int32_t num_ops, fm_plan *const *plans,
              (ls0.kind == 6 && ls0.rc_L >= 128))) {
           rxmode = ls0.kind == 5 ? fmk::RXM_FFT : fmk::RXM_CONV;
           rx = rx_step(ls0, st);
-          const i64 per = fmk::kRxbPoints / ls0.rc_L;
-          tiles = ls0.kind == 5 ? (st.V + per - 1) / per * M
-                                : (st.V * M + per - 1) / per;
+          // an FFT tile is one or two groups of adjacent vectors of a
+          // column, a convolution tile any consecutive vectors
+          const int L = ls0.rc_L;
+          const i64 nv = ls0.kind == 5 ? fmk::rxb_nv(L)
+                                       : fmk::kRxbPoints / L;
+          const i64 per = ls0.kind == 5
+                              ? FM_MAX_THREADS / fmk::rxb_group(L)
+                              : 1;
+          const i64 groups = ls0.kind == 5 ? (st.V + nv - 1) / nv * M
+                                           : (st.V * M + nv - 1) / nv;
+          tiles = (groups + per - 1) / per;
         }
         // the batch kernel has no class 5: its class 1 runs the same
         // program with the spectrum product as a separate op

@@ -198,10 +198,22 @@ __device__ __forceinline__ int rc_off(int j) {  // register j = u R + r
   return (j / R) * G * R + M * (j % R);
 }
 
+// Barrier of the threads that exchange points: SY = 0 one warp, 1 the CTA,
+// SY >= 64 aligned groups of SY threads (named barriers 1 + group)
+template <int SY> __device__ __forceinline__ void rc_sync() {
+  if constexpr (SY == 0)
+    __syncwarp();
+  else if constexpr (SY == 1)
+    __syncthreads();
+  else
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)(threadIdx.x / SY)),
+                 "n"(SY)
+                 : "memory");
+}
+
 // Registers laid out for stage IA -> shared buffer -> registers laid out
-// for stage IB (warp barriers: the lanes of a vector are in one warp).
-// (CTA: the threads of a vector span several warps, CTA barriers)
-template <class E, int L, int IA, int IB, bool CTA = false>
+// for stage IB.
+template <class E, int L, int IA, int IB, int SY = 0>
 __device__ __forceinline__ void rc_exchange(E (&x)[RcLane<E>::P], E *buf,
                                             int g) {
   constexpr int P = RcLane<E>::P;
@@ -213,27 +225,20 @@ __device__ __forceinline__ void rc_exchange(E (&x)[RcLane<E>::P], E *buf,
   const E *const ra = buf + rc_pad<E, L>(rc_base<E, L, IB>(g));
 #pragma unroll
   for (int j = 0; j < P; ++j) wa[rc_pad<E, L>(rc_off<E, L, IA>(j))] = x[j];
-  if constexpr (CTA)
-    __syncthreads();
-  else
-    __syncwarp();
+  rc_sync<SY>();
 #pragma unroll
   for (int j = 0; j < P; ++j) x[j] = ra[rc_pad<E, L>(rc_off<E, L, IB>(j))];
-  if constexpr (CTA)
-    __syncthreads();
-  else
-    __syncwarp();
+  rc_sync<SY>();
 }
 
-template <class E, int L, int I, int FSG = -1, bool CTA = false,
-          bool GT = false>
+template <class E, int L, int I, int FSG = -1, int SY = 0, bool GT = false>
 __device__ __forceinline__ void rc_forward(E (&x)[RcLane<E>::P], E *buf, int g,
                                            const E *stw) {
   rc_stage<E, L, I, false, FSG, GT>(x, g, stw);
   constexpr int S = rc_stages(L, RcLane<E>::P);
   if constexpr (I + 1 < S) {
-    rc_exchange<E, L, I, I + 1, CTA>(x, buf, g);
-    rc_forward<E, L, I + 1, FSG, CTA, GT>(x, buf, g, stw);
+    rc_exchange<E, L, I, I + 1, SY>(x, buf, g);
+    rc_forward<E, L, I + 1, FSG, SY, GT>(x, buf, g, stw);
   }
 }
 
@@ -264,13 +269,13 @@ template <class E, int L>
 __device__ __forceinline__ int rc_nat(int p) {
   return rc_nat_from<E, L, 0>(p, 0);
 }
-template <class E, int L, int I, bool CTA = false, bool GT = false>
+template <class E, int L, int I, int SY = 0, bool GT = false>
 __device__ __forceinline__ void rc_inverse(E (&x)[RcLane<E>::P], E *buf, int g,
                                            const E *stw) {
   rc_stage<E, L, I, true, -1, GT>(x, g, stw);
   if constexpr (I > 0) {
-    rc_exchange<E, L, I, I - 1, CTA>(x, buf, g);
-    rc_inverse<E, L, I - 1, CTA, GT>(x, buf, g, stw);
+    rc_exchange<E, L, I, I - 1, SY>(x, buf, g);
+    rc_inverse<E, L, I - 1, SY, GT>(x, buf, g, stw);
   }
 }
 

@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(RxShape<E, L>::TF,
     rx_pre<E, L>(x, p, act, rb, t, G);
     // (S >= 2: the exchanges' barriers also separate this batch's reads of
     // sexp from the next batch's reset)
-    rc_forward<E, L, 0, -1, true, true>(x, buf, t, (const E *)p.tw);
+    rc_forward<E, L, 0, -1, 1, true>(x, buf, t, (const E *)p.tw);
     if (act) {
       const unsigned ao = dO.div(v), co = v - ao * (unsigned)p.out_cc;
       // register u R + r holds natural index jn + u R + r L / R
@@ -481,14 +481,14 @@ __global__ void __launch_bounds__(RxShape<E, L>::TC,
       for (int r = 0; r < P; ++r) x[r] = E{d[r].x, d[r].y};
     }
     rx_pre<E, L>(x, p, act, rb, g, G);
-    rc_forward<E, L, 0, -1, CTA, true>(x, buf, g, (const E *)p.tw);
+    rc_forward<E, L, 0, -1, CTA ? 1 : 0, true>(x, buf, g, (const E *)p.tw);
     if (act) {
       const E *sp = (const E *)p.spec + (i64)v * p.spec_stride + g;
 #pragma unroll
       for (int j = 0; j < P; ++j)
         x[j] = mulv(x[j], tw_get<true>(sp, j * G), p.spec_conj != 0);
     }
-    rc_inverse<E, L, S - 1, CTA, true>(x, buf, g, (const E *)p.tw);
+    rc_inverse<E, L, S - 1, CTA ? 1 : 0, true>(x, buf, g, (const E *)p.tw);
     if (act)
       rx_store<E, L>(x, s, p, v, (i64)m * p.ld_dst, (i64)v * p.out_n, g,
                      [](int r) { return G * r; });

@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(RsfShape<E, L>::T, (RsfOcc<E>::v))
     }
     // (S >= 2: the stages hold at least one exchange, whose barriers also
     // separate this batch's reads of sexp from the next batch's reset)
-    rc_forward<E, L, 0, SG, true>(x, buf, t, stw);
+    rc_forward<E, L, 0, SG, 1>(x, buf, t, stw);
     // register u R + r of the last stage (radix R) holds the natural index
     // of the thread's base plus u R + r L / R
     constexpr int R = rc_radix(S - 1, L, P);
