@@ -320,7 +320,9 @@ __global__ void __launch_bounds__(RfShape<E, L>::T, (RfOcc<E, L>::v))
 template <class E, int L> struct RsShape {
   static constexpr int P = RfLane<E>::P;
   static constexpr int W = L / P;             // threads per vector
-  static constexpr int NV = W > 32 ? 16 : 32;  // vectors per CTA batch
+  // vectors per CTA batch (rows of 128 bytes; float64 at 32 vectors, twice
+  // the threads, leaves room for fewer registers or CTAs)
+  static constexpr int NV = W > 32 || RfLane<E>::fixed ? 16 : 32;
   static constexpr int T = NV * W;
   static constexpr int Lx = (L + (L >> RfLane<E>::XSH)) | 1;
 };
@@ -330,8 +332,12 @@ __host__ __device__ constexpr size_t rs_smem() {
          32 * sizeof(int);
 }
 template <class E, int L> struct RsOcc {
-  static constexpr int v =
-      RsShape<E, L>::T >= 1024 ? 1 : 1024 / RsShape<E, L>::T;
+  // (fixed point up to 256 points: 80 registers a thread, 64 spill: the
+  // FWHT mode of Kron(F256, H8, C128) on 8 columns 534 -> 449 us with this
+  // and 16 vectors a CTA)
+  static constexpr int T = RsShape<E, L>::T;
+  static constexpr int B = RfLane<E>::fixed && T <= 256 ? 768 : 1024;
+  static constexpr int v = T >= B ? 1 : B / T;
 };
 
 // One batch bt of NV adjacent strided vectors (NV = 32, 16, ..., the
