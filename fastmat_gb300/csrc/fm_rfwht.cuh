@@ -135,6 +135,22 @@ __device__ __forceinline__ void rf_levels(LE (&v)[P]) {
     for (int h = 1; h < R; h <<= 1) {
 #pragma unroll
       for (int r = 0; r < R; ++r) {
+        if constexpr (std::is_same<LE, float>::value) {
+          // pairs of adjacent points in one packed operation
+          if (h >= 2) {
+            if ((r & (h | 1)) == 0) {
+              const int i = u * R + r;
+              const float2 a = make_float2(v[i], v[i + 1]);
+              const float2 c = make_float2(v[i + h], v[i + h + 1]);
+              const float2 p = add2(a, c), q = sub2(a, c);
+              v[i] = p.x;
+              v[i + 1] = p.y;
+              v[i + h] = q.x;
+              v[i + h + 1] = q.y;
+            }
+            continue;
+          }
+        }
         if ((r & h) == 0) {
           const LE a = v[u * R + r], c = v[u * R + r + h];
           v[u * R + r] = addv(a, c);

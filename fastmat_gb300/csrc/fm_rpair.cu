@@ -10,6 +10,9 @@
 
 namespace fmk {
 
+// complex64 with packed additions, 16 points a thread
+typedef cfp<16> cf16;
+
 namespace {
 
 template <class E, int L1, int L2>
@@ -80,10 +83,10 @@ bool rkch_supported(int ctype, int L1, int L2, i64 block_rows,
     return fits<E, A, B>(block_rows, real_per_block) &&                   \
            set(RchShape<E, A, B>::VPC, RchShape<E, A, B>::NV2);
   if (ctype == FM_C64) {
-    FM_RCH_CASE(float2, 128, 128)
-    FM_RCH_CASE(float2, 128, 256)
-    FM_RCH_CASE(float2, 256, 128)
-    FM_RCH_CASE(float2, 256, 256)
+    FM_RCH_CASE(cf16, 128, 128)
+    FM_RCH_CASE(cf16, 128, 256)
+    FM_RCH_CASE(cf16, 256, 128)
+    FM_RCH_CASE(cf16, 256, 256)
   }
 #undef FM_RCH_CASE
   return false;
@@ -94,10 +97,10 @@ cudaError_t launch_rkch(int ctype, const RchPair &p, cudaStream_t s) {
 #define FM_RCH_LAUNCH(E, A, B) \
   if (L1 == A && L2 == B) return launch_one<E, A, B>(p, s);
   if (ctype == FM_C64) {
-    FM_RCH_LAUNCH(float2, 128, 128)
-    FM_RCH_LAUNCH(float2, 128, 256)
-    FM_RCH_LAUNCH(float2, 256, 128)
-    FM_RCH_LAUNCH(float2, 256, 256)
+    FM_RCH_LAUNCH(cf16, 128, 128)
+    FM_RCH_LAUNCH(cf16, 128, 256)
+    FM_RCH_LAUNCH(cf16, 256, 128)
+    FM_RCH_LAUNCH(cf16, 256, 256)
   }
 #undef FM_RCH_LAUNCH
   return cudaErrorInvalidConfiguration;

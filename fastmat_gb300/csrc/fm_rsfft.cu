@@ -64,11 +64,11 @@ int rsfft_max_len(int ctype) {
 cudaError_t launch_rsfft(int ctype, const RsfStep &p, cudaStream_t s) {
   if (ctype == FM_C64) {
     switch (p.L) {
-      case 32: return launch_signed<float2, 32>(p, s);
-      case 64: return launch_signed<float2, 64>(p, s);
-      case 128: return launch_signed<float2, 128>(p, s);
-      case 256: return launch_signed<float2, 256>(p, s);
-      case 512: return launch_signed<float2, 512>(p, s);
+      case 32: return launch_signed<cfp<16>, 32>(p, s);
+      case 64: return launch_signed<cfp<16>, 64>(p, s);
+      case 128: return launch_signed<cfp<16>, 128>(p, s);
+      case 256: return launch_signed<cfp<16>, 256>(p, s);
+      case 512: return launch_signed<cfp<16>, 512>(p, s);
       default: break;
     }
   } else if (ctype == FM_C128_DF) {

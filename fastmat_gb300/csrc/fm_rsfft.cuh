@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(RsfShape<E, L>::T, (RsfOcc<E>::v))
   constexpr int P = Sh::P, G = Sh::G, NV = Sh::NV;
   constexpr int S = rc_stages(L, P);
   static_assert(G >= 2 && NV >= 1 && NV <= 32, "vector layout");
-  typedef typename std::conditional<Emu<E>::v, double2, E>::type Raw;
+  typedef typename std::conditional<Emu<E>::v, double2, float2>::type Raw;
   extern __shared__ __align__(128) unsigned char fm_smem[];
   constexpr int TWN = rc_twlen<E, L, S>();
   E *stw = reinterpret_cast<E *>(fm_smem);
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(RsfShape<E, L>::T, (RsfOcc<E>::v))
       rx_in<P>(x, d, s);
     } else {
 #pragma unroll
-      for (int r = 0; r < P; ++r) x[r] = d[r];
+      for (int r = 0; r < P; ++r) x[r] = E{d[r].x, d[r].y};
     }
     // (S >= 2: the stages hold at least one exchange, whose barriers also
     // separate this batch's reads of sexp from the next batch's reset)
