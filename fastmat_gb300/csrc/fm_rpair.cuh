@@ -100,12 +100,18 @@ __global__ void __launch_bounds__(FM_RCH_THREADS, (RchOcc<E>::v))
   const unsigned nb = NB > lag ? NB - lag : 0u;
   const FDiv dAc((unsigned)p.c.A), dAh((unsigned)p.h.A),
       dSh((unsigned)p.h.es);
-  for (;;) {
-    if (tid == 0) sitem[0] = atomicAdd(p.ctr, 1u);
-    __syncthreads();
-    const unsigned item = sitem[0];
-    __syncthreads();  // (sitem is rewritten by the next item)
+  // The next item is taken while the current one runs, so that the counter's
+  // round trip is covered (a FWHT item still waits only for items
+  // handed out before it: the unfinished convolution item with the smallest
+  // number is running, or waiting behind an item with a smaller number,
+  // whose own convolution items have all finished)
+  if (tid == 0) sitem[0] = atomicAdd(p.ctr, 1u);
+  __syncthreads();
+  for (int par = 0;; par ^= 1) {
+    const unsigned item = sitem[par];
     if (item >= total) break;
+    unsigned next = 0;
+    if (tid == 0) next = atomicAdd(p.ctr, 1u);
     // block k's convolution items, then block k - lag's FWHT items (the
     // first lag blocks' convolutions alone, the last lag blocks' FWHTs at
     // the end)
@@ -152,7 +158,9 @@ __global__ void __launch_bounds__(FM_RCH_THREADS, (RchOcc<E>::v))
                  (i64)a * p.c.out_stride;
 #pragma unroll
       for (int r = 0; r < P; ++r) dst[g + G * r] = x[r];
-      // this item's stores, then its count (release)
+      // this item's stores, then its count (release); the barrier also
+      // frees the shared memory for the next item
+      if (tid == 0) sitem[par ^ 1] = next;
       __syncthreads();
       if (tid == 0) {
         __threadfence();
@@ -160,6 +168,7 @@ __global__ void __launch_bounds__(FM_RCH_THREADS, (RchOcc<E>::v))
       }
     } else {
       // wait for the block's convolution items (acquire), bounded
+      bool ok = true;
       if (tid == 0) {
         long long polls = 0;
         unsigned done;
@@ -175,18 +184,16 @@ __global__ void __launch_bounds__(FM_RCH_THREADS, (RchOcc<E>::v))
           }
           __nanosleep(64);
         }
-        sitem[1] = done >= n1 ? 1u : 0u;
+        ok = done >= n1;
+        sitem[par ^ 1] = next;
       }
-      __syncthreads();
-      const bool ready = sitem[1] != 0;
-      __syncthreads();
-      if (ready) {
+      if (__syncthreads_and(ok)) {
         R *xb = reinterpret_cast<R *>(region);
         int *sexp = reinterpret_cast<int *>(xb + NV2 * RsShape<R, L2>::Lx);
         rs_batch<R, L2, NV2>(p.h, (i64)blk * n2 + idx, xb, sexp, dAh, dSh);
       }
+      __syncthreads();  // shared memory is reused by the next item
     }
-    __syncthreads();  // shared memory is reused by the next item
   }
 }
 
