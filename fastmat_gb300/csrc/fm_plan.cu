@@ -2612,7 +2612,7 @@ void launch_step(fm_plan *P, LStep &ls, fmk::Step &st, cudaStream_t s) {
       if (rf.A * rf.num_cols >= 0x7fffffffLL || rf.es >= 0x7fffffffLL)
         fail(FM_ERR_UNSUPPORTED, "more than 2^31 vectors in one launch");
       if (ls.pair == 1 && !P->no_pair && 1 + st.num_cols <= P->pair_cap &&
-          (i64)st.num_cols * (rf.A + ls.rc2_A) < 0xffffffffLL) {
+          (i64)st.num_cols * (rf.A + ls.rc2_A) < 0xffff0000LL) {
         // both passes, column by column; the second runs in place on dst
         fmk::RfPair pr;
         pr.a = rf;
@@ -2625,7 +2625,7 @@ void launch_step(fm_plan *P, LStep &ls, fmk::Step &st, cudaStream_t s) {
         pr.ctr = P->pair_ctr;
         pr.err = P->err;
         pr.wait_limit = P->wait_limit;
-        pr.lag = 1;  // (2 for float32 measured slower: 0.72 vs 0.67 ms)
+        pr.lag = 1;  // set by the launcher from the resident grid
         CUDA_TRY(cudaMemsetAsync(P->pair_ctr, 0,
                                  (size_t)(1 + st.num_cols) * 4, s));
         CUDA_TRY(fmk::launch_rfwht2(ls.rc_ct, pr, s));
@@ -2707,7 +2707,7 @@ void launch_step(fm_plan *P, LStep &ls, fmk::Step &st, cudaStream_t s) {
     const i64 blocks = (i64)ls.rc2_blocks * st.num_cols;
     if (ls.pair == 3 && !P->no_pair && st.src_type == P->io_type &&
         st.dst_type == P->io_type && 1 + blocks <= P->pair_cap &&
-        blocks * (ls.rc2_n1 + ls.rc2_n2) < 0xffffffffLL &&
+        blocks * (ls.rc2_n1 + ls.rc2_n2) < 0xffff0000LL &&
         ls.rc2_A * st.num_cols < 0x7fffffffLL) {
       // this circulant mode and the Hadamard mode after it, block by block;
       // the FWHT runs in place on dst, in its real view (two real words
