@@ -350,15 +350,36 @@ template <int R> __host__ __device__ constexpr int brev(int i) {
 // Unsigned division by a runtime divisor 1 <= d < 2^31 for dividends below
 // 2^31 with one multiply-high: q = (umulhi(n, m) + n) >> s,
 // s = ceil(log2 d), m = 2^32 (2^s - d) / d + 1 (round-up multiplier).
-// Powers of two (the common case: built per FFT stage of every tile) skip
-// the 64-bit division: m = 1, and umulhi(n, 1) = 0 leaves n >> s.
+// Powers of two (the common case: built per FFT stage of every tile) have
+// m = 1, and umulhi(n, 1) = 0 leaves n >> s.  For other divisors the quotient
+// of m is estimated in float (within 2^10) and corrected by its remainder: a
+// 64-bit division takes the FP64 pipe, the slowest of this GPU (Fourier(6000)
+// x 64, 9 of them a launch: 15 % of its cycles busy there).
 struct FDiv {
   unsigned d, m, s;
   __device__ __forceinline__ explicit FDiv(unsigned d_) : d(d_) {
     s = d > 1 ? 32 - __clz(d - 1) : 0;  // ceil(log2 d)
-    m = (d & (d - 1)) == 0
-            ? 1u
-            : (unsigned)(((1ull << 32) * ((1ull << s) - d)) / d + 1);
+    m = 1u;
+    if (d & (d - 1)) {
+      const unsigned e = (1u << s) - d;
+      const float fd = (float)d;
+      const float est = __fdiv_rn((float)e, fd) * 4294967296.f;
+      unsigned q = (unsigned)fminf(est, 4294967040.f);
+      i64 rem = (i64)(((unsigned long long)e << 32) -
+                      (unsigned long long)q * d);
+      // |rem| <= 2^10 d: exact below 2^20 d, else to 16 bits more than enough
+      const float t = d < (1u << 20) ? (float)(int)rem
+                                     : (float)(int)(rem >> 16) * 65536.f;
+      const int c = __float2int_rd(__fdiv_rn(t, fd));
+      q += (unsigned)c;
+      rem -= (i64)c * (i64)d;
+      if (rem < 0) {
+        --q;
+        rem += d;
+      }
+      if (rem >= (i64)d) ++q;
+      m = q + 1u;
+    }
   }
   __device__ __forceinline__ unsigned div(unsigned n) const {
     return (__umulhi(n, m) + n) >> s;
@@ -1241,7 +1262,8 @@ __device__ __forceinline__ void store_fixup_vm(const Step &p, E *sm,
   if (!any) return;
   const E *post = (const E *)p.post;
   const bool has_scale = p.has_scale != 0, cj = p.conj_out != 0;
-  const E c = scalar_of<E>(p.scale_re, p.scale_im);
+  // (float64 -> float conversions take the FP64 pipe)
+  const E c = p.has_scale ? scalar_of<E>(p.scale_re, p.scale_im) : zero<E>();
   Walk w(tid, n, T);
   for (int f = tid; f < total; f += T, w.next()) {
     const int b = w.b, j = w.j;
@@ -1438,7 +1460,8 @@ __device__ __forceinline__ void store_fixup_em(const Step &p, E *sm,
     __syncthreads();
   }
   if (!p.post && !p.has_scale && !p.conj_out) return;
-  const E c = scalar_of<E>(p.scale_re, p.scale_im);
+  // (float64 -> float conversions take the FP64 pipe)
+  const E c = p.has_scale ? scalar_of<E>(p.scale_re, p.scale_im) : zero<E>();
   for (int f = tid; f < total; f += T) {
     const int b = f & (B - 1), j = f >> lgB;
     E val = sm[f];
@@ -1460,7 +1483,8 @@ __device__ __forceinline__ void store_tile(const Step &p, const E *sm,
                                            bool natural = false) {
   const int B = p.B, Lp = p.Lp;
   const bool acc = p.accumulate != 0;
-  const E c = scalar_of<E>(p.scale_re, p.scale_im);
+  // (float64 -> float conversions take the FP64 pipe)
+  const E c = p.has_scale ? scalar_of<E>(p.scale_re, p.scale_im) : zero<E>();
   if constexpr (LAY != 1) {
     if (p.out_mode == 1) {
       // gather: out row i of column m takes vector element map_out[i]
@@ -1722,7 +1746,7 @@ __global__ void __launch_bounds__(FM_MAX_THREADS, (MinBlocks<E, CLS>::v))
   auto buf = [&](int k) { return reinterpret_cast<E *>(fm_smem + k * tb); };
   auto vis = [&](int k) { return vi0 + k * B; };
   const i64 nvec = p.V * p.num_cols;
-  const i64 ntiles = (nvec + B - 1) / B;
+  const i64 ntiles = (nvec + B - 1) >> (__ffs(B) - 1);  // (B = 2^k)
   const FDiv dV((unsigned)p.V), dci((unsigned)p.vin.Cc),
       dco((unsigned)p.vout.Cc);
   const bool tma_in = p.tma_in != 0;    // hardware copies into the ring
