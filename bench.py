@@ -370,6 +370,8 @@ def roofline_of(fg, plan, per_launch, n_in, n_out, M, dt, out_dt, peak,
         kernel = 'rfwht' if 'stride=1 ' in line else 'rsfwht'
     elif 'rsfft' in line:
         kernel = 'rsfft'
+    elif ' rxconv ' in line or ' rxfft ' in line:
+        kernel = 'rxconv' if ' rxconv ' in line else 'rxfft'
     else:
         kernel = what
     return {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
