@@ -9,6 +9,14 @@
 // of fm_rfft.cuh take a tile's points, copied ahead, into registers,
 // transform and store them directly, 8 points on each of the CTA's 512
 // threads.
+// 64 operators of 64..65536 points: 425 -> 327 us with direct loads, 321
+// with the points copied ahead, 309 with barriers of the threads that
+// exchange only.  Per tile they still take 1.7 times what the separate
+// launches of fm_rfft.cuh take: 64 registers hold the records' fields and
+// the transform, barriers and load latency lead the stalls.  Measured and
+// left out: one CTA of 128 registers a thread (385 us), runs of one step's
+// tiles without CTA barriers and with host-made divisors (312), all factors
+// of a product loaded before use (323: spills).
 #pragma once
 
 #include "fm_rfft.cuh"

@@ -283,9 +283,11 @@ __device__ __forceinline__ void rc_inverse(E (&x)[RcLane<E>::P], E *buf, int g,
 // pipe (Kron(F256, H8, C128), 8 columns, before: 0.62 issued per cycle, ALU
 // 48 %, FMA 37 %): packed arithmetic (one instruction for both parts) and
 // the conversions below (13 + 19 instead of about 15 + 31 instructions per
-// real word, no FP64 addition) took its step from 3.70 to 2.61 ms.  (A
-// barrier per batch to keep the warps of a CTA on the same instructions
-// measured 2.62 ms and is left out.)
+// real word, no FP64 addition) took its step from 3.70 to 2.61 ms, this
+// kernel's launch from 1850 to 1015 us; the FMA pipe is now 74 % busy (about
+// 410 FP32 operations per element, 720 us at its full rate).  (A barrier per
+// batch to keep the warps of a CTA on the same instructions measured 2.62 ms
+// for the step and is left out.)
 // ---- raw points of a double-float vector (complex128 words) and the
 // registers of the transforms; single precision passes through
 template <int P>

@@ -31,13 +31,20 @@
 // Measured against the stage kernel's tiles (vprog_kernel, every radix stage
 // a pass over shared memory with run-time index arithmetic), microseconds
 // per launch: 32 columns of 2^18 points, double-float, strided 512 points
-// 347 -> 168, convolution of 512 points 558 -> 183; the same in complex64
-// 118 -> 38 and 62 -> 38; convolution of 4096 points, 4 columns,
-// double-float 57 -> 19.  Eight points a thread in complex64 too: 16 (the
-// radices 16, 16, 2) measured 6 % further from 64-bit results over 2^18
-// points, and spilled in the convolution.  The double-float launches are
-// bound by instruction issue, the complex64 ones by the load and exchange
-// latencies of one batch (their operands stay in L2).
+// 347 -> 134 (with gathers and products around), convolution of 512 points
+// 558 -> 185; the same in complex64 118 -> 35 and 62 -> 43; convolution of
+// 4096 points, 4 columns, double-float 57 -> 19.  Eight points a thread in
+// complex64 too: 16 (the radices 16, 16, 2) measured 6 % further from 64-bit
+// results over 2^18 points, and spilled in the convolution.  The next batch
+// is copied ahead (strided complex64 38 -> 35, gathered double-float 168 ->
+// 134).  Bounds: the FMA pipe in double-float (67 % busy in the convolution,
+// 47 % in the FFT passes, whose table loads and barriers 16 warps a
+// multiprocessor do not cover), the shared-memory / L1 pipe in complex64 (50
+// to 69 %).  Measured and left out, in double-float: intermediates as packed
+// double-floats instead of float64 words (no change: the conversions run in
+// the integer pipe's spare cycles), half the vectors a CTA (2^18 x 32 chain
+// 463 -> 478 us), 96 registers a thread (convolution 185 -> 196), barriers
+// per vector (185 -> 188).
 #pragma once
 
 #include <map>

@@ -4,7 +4,10 @@
 // data (64-bit fixed point, see fx in fm_types.cuh: float64 launches were
 // bound by the double-float additions and conversions; Hadamard(18) on 48
 // columns 224 -> 129 us, the FWHT mode of Kron(F256, H8, C128) on 8 complex
-// columns 875 -> 540 us, errors against 64 bits 7.2e-15 -> 1.3e-15).
+// columns 875 -> 532 us, errors against 64 bits 7.2e-15 -> 1.3e-15; 99.5 and
+// 451 us with the later changes below).  The float64 kernels are bound by the
+// integer pipe (66 % busy in the strided one), the float32 ones by barriers
+// and the shared-memory pipe (55-60 % busy).
 //
 //   * a vector of L points is held by G = L / P threads of a CTA, P points
 //     per thread (32 float or 16 fixed-point); the CTA works on
@@ -431,7 +434,7 @@ __global__ void __launch_bounds__(RsShape<E, L>::T, (RsOcc<E, L>::v))
 // by the second) is still in L2 when the second pass reads it.  Work items
 // are handed out in order by an atomic counter: the first-pass items of
 // column k (one vector each), then the second-pass items of column k - lag
-// (NV2 strided vectors each; the planner uses lag 1).  A second-pass item of column m waits until
+// (NV2 strided vectors each; the launcher sets the lag).  A second-pass item of column m waits until
 // all first-pass items of column m have finished (their count in ctr[1 +
 // m], raised with release semantics after each item's stores; read with
 // acquire semantics, polls bounded by wait_limit).  Every awaited item was

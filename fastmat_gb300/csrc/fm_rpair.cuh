@@ -104,7 +104,8 @@ __global__ void __launch_bounds__(FM_RCH_THREADS, (RchOcc<E>::v))
   // round trip is covered (a FWHT item still waits only for items
   // handed out before it: the unfinished convolution item with the smallest
   // number is running, or waiting behind an item with a smaller number,
-  // whose own convolution items have all finished)
+  // whose own convolution items have all finished).  Kron(F256, H8, C128) on
+  // 8 columns, both launches: 499 -> 485 us.
   if (tid == 0) sitem[0] = atomicAdd(p.ctr, 1u);
   __syncthreads();
   for (int par = 0;; par ^= 1) {
