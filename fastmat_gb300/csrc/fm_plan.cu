@@ -1987,11 +1987,15 @@ class Planner {
   // circular convolution of contiguous vectors (kind 6), with the loader's
   // and storer's work around it and an optional four-step twiddle at its
   // end, runs in the register transforms of long vectors when its length is
-  // a power of two they are built for.  Lines of the rule: strided vectors
-  // need rows of at least 64 bytes (two sectors; narrower ones load no
-  // better there than in the stage kernel's tiles); a plain Fourier mode of
-  // a Kron above 512 points, and a whole Fourier column in one launch, stay
-  // on the stage kernel's tiles.
+  // a power of two they are built for.  Lines of the rule: rows of two or
+  // more adjacent vectors (a Fourier mode of 256 points, 2^20 x 8: at 2
+  // vectors a row 88 us on the stage kernel's tiles, 49 here in complex64, 214
+  // and 109 in double-float; at 8 vectors 76 and 32, 200 and 101; whole
+  // convolutions of 4096 points, 256 columns in double-float, 112 and 40).
+  // A plain Fourier mode of a Kron above 512 points, and a whole Fourier
+  // column in one launch, stay on the stage kernel's tiles, whose copies the
+  // plan's wait limit bounds (1024 points at stride 64, complex64: 74 us
+  // there, 50 here).
   void try_rx(LStep &ls, const std::vector<fmk::Op> &ops) {
     const int ct = P_->ctype;
     if (ct != FM_C64 && ct != FM_C128_DF) return;
@@ -2048,7 +2052,7 @@ class Planner {
         (cj_out && st.conj_out))
       return;
     const i64 ci = st.vin.Cc, co = st.vout.Cc;
-    const i64 wide = 64 / P_->esz;
+    const i64 wide = 2;  // vectors in a row
     if (sm) {
       if (ci != 1 || co != 1 || L < fmk::rxconv_min || L > fmk::rxconv_max)
         return;

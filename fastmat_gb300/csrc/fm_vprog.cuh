@@ -1262,8 +1262,7 @@ __device__ __forceinline__ void store_fixup_vm(const Step &p, E *sm,
   if (!any) return;
   const E *post = (const E *)p.post;
   const bool has_scale = p.has_scale != 0, cj = p.conj_out != 0;
-  // (float64 -> float conversions take the FP64 pipe)
-  const E c = p.has_scale ? scalar_of<E>(p.scale_re, p.scale_im) : zero<E>();
+  const E c = scalar_of<E>(p.scale_re, p.scale_im);
   Walk w(tid, n, T);
   for (int f = tid; f < total; f += T, w.next()) {
     const int b = w.b, j = w.j;
@@ -1460,8 +1459,7 @@ __device__ __forceinline__ void store_fixup_em(const Step &p, E *sm,
     __syncthreads();
   }
   if (!p.post && !p.has_scale && !p.conj_out) return;
-  // (float64 -> float conversions take the FP64 pipe)
-  const E c = p.has_scale ? scalar_of<E>(p.scale_re, p.scale_im) : zero<E>();
+  const E c = scalar_of<E>(p.scale_re, p.scale_im);
   for (int f = tid; f < total; f += T) {
     const int b = f & (B - 1), j = f >> lgB;
     E val = sm[f];
@@ -1483,8 +1481,7 @@ __device__ __forceinline__ void store_tile(const Step &p, const E *sm,
                                            bool natural = false) {
   const int B = p.B, Lp = p.Lp;
   const bool acc = p.accumulate != 0;
-  // (float64 -> float conversions take the FP64 pipe)
-  const E c = p.has_scale ? scalar_of<E>(p.scale_re, p.scale_im) : zero<E>();
+  const E c = scalar_of<E>(p.scale_re, p.scale_im);
   if constexpr (LAY != 1) {
     if (p.out_mode == 1) {
       // gather: out row i of column m takes vector element map_out[i]
@@ -1746,7 +1743,7 @@ __global__ void __launch_bounds__(FM_MAX_THREADS, (MinBlocks<E, CLS>::v))
   auto buf = [&](int k) { return reinterpret_cast<E *>(fm_smem + k * tb); };
   auto vis = [&](int k) { return vi0 + k * B; };
   const i64 nvec = p.V * p.num_cols;
-  const i64 ntiles = (nvec + B - 1) >> (__ffs(B) - 1);  // (B = 2^k)
+  const i64 ntiles = (nvec + B - 1) / B;
   const FDiv dV((unsigned)p.V), dci((unsigned)p.vin.Cc),
       dco((unsigned)p.vout.Cc);
   const bool tma_in = p.tma_in != 0;    // hardware copies into the ring

@@ -134,7 +134,7 @@ def test_chain_sum_conjugate(n, prec, dt, tol):
 
 @pytest.mark.parametrize('prec,dt,tol', PREC)
 @pytest.mark.parametrize('L', [32, 64, 128, 256, 512])
-@pytest.mark.parametrize('inner', [9, 24, 33])
+@pytest.mark.parametrize('inner', [2, 3, 9, 24, 33])
 def test_strided_mode_with_ragged_stride(L, inner, prec, dt, tol):
     """A Fourier mode of a Kron at a stride that is no multiple of 32."""
     import fastmat_gb300 as fm
