@@ -1,7 +1,7 @@
 // Launcher of the batched persistent kernel (many operators in one
 // cooperative launch; see batch_kernel in fm_batch.cuh).  The instantiations
-// live in translation units of their own (fm_batch_c64.cu,
-// fm_batch_c64_gen.cu, fm_batch_df.cu), which compile in parallel.
+// live in translation units of their own (fm_batch_c64_pow2.cu,
+// fm_batch_c64.cu, fm_batch_c64_gen.cu, fm_batch_df.cu), which compile in parallel.
 
 #include <cuda_runtime.h>
 
@@ -10,6 +10,7 @@
 
 namespace fmk {
 
+cudaError_t launch_batch_c64_pow2(const BatchLaunch &b, cudaStream_t s);
 cudaError_t launch_batch_c64(const BatchLaunch &b, cudaStream_t s);
 cudaError_t launch_batch_c64_gen(const BatchLaunch &b, cudaStream_t s);
 cudaError_t launch_batch_df(const BatchLaunch &b, cudaStream_t s);
@@ -17,9 +18,9 @@ cudaError_t launch_batch_df(const BatchLaunch &b, cudaStream_t s);
 cudaError_t launch_batch(const BatchLaunch &b, cudaStream_t s) {
   switch (b.ctype) {
     case FM_C64:
-      // class 2 covers class 1's programs (power-of-two FFTs only)
-      return b.cls == 1 || b.cls == 2 ? launch_batch_c64(b, s)
-                                      : launch_batch_c64_gen(b, s);
+      return b.cls == 1   ? launch_batch_c64_pow2(b, s)
+             : b.cls == 2 ? launch_batch_c64(b, s)
+                          : launch_batch_c64_gen(b, s);
     case FM_C128_DF: return launch_batch_df(b, s);
     default: return cudaErrorNotSupported;
   }
