@@ -257,7 +257,7 @@ __device__ __forceinline__ void batch_issue_load(const Step *gp, Step *slot,
   __syncthreads();
   const Step &p = *slot;
   const i64 nvec = p.V * p.num_cols;
-  const FDiv dV((unsigned)p.V), dci((unsigned)p.vin.Cc),
+  const FDivF dV((unsigned)p.V), dci((unsigned)p.vin.Cc),
       dco((unsigned)p.vout.Cc);
   setup_tile(p, vi, tile, dV, dci, dco, nvec, tid, T);
   __syncthreads();

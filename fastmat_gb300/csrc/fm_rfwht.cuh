@@ -225,7 +225,7 @@ template <class E, int L> __host__ __device__ constexpr int rf_last() {
 template <class E, int L>
 __device__ __forceinline__ void rf_finish(
     typename RfShape<E, L>::Raw (&d)[RfLane<E>::P], const RfStep &p, i64 gv,
-    bool act, E *buf, int *sexp, int vl, int t, const FDiv &dA) {
+    bool act, E *buf, int *sexp, int vl, int t, const FDivB &dA) {
   typedef RfShape<E, L> Sh;
   constexpr int P = Sh::P, G = Sh::G, VPC = Sh::VPC;
   constexpr int SL = rf_last<E, L>();
@@ -363,8 +363,8 @@ template <class E, int L> struct RsOcc {
 // launch's threads / (L / P)): thread t = tid / NV of vector v = tid % NV.
 template <class E, int L, int NV>
 __device__ __forceinline__ void rs_batch(const RfStep &p, i64 bt, E *xb,
-                                         int *sexp, const FDiv &dA,
-                                         const FDiv &dS) {
+                                         int *sexp, const FDivB &dA,
+                                         const FDivB &dS) {
   typedef typename RfLane<E>::Raw Raw;
   constexpr int P = RfLane<E>::P, W = L / P;
   constexpr int Lx = RsShape<E, L>::Lx;

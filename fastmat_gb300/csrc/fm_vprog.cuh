@@ -351,13 +351,32 @@ template <int R> __host__ __device__ constexpr int brev(int i) {
 // 2^31 with one multiply-high: q = (umulhi(n, m) + n) >> s,
 // s = ceil(log2 d), m = 2^32 (2^s - d) / d + 1 (round-up multiplier).
 // Powers of two (the common case: built per FFT stage of every tile) have
-// m = 1, and umulhi(n, 1) = 0 leaves n >> s.  For other divisors the quotient
-// of m is estimated in float (within 2^10) and corrected by its remainder: a
-// 64-bit division takes the FP64 pipe, the slowest of this GPU (Fourier(6000)
-// x 64, 9 of them a launch: 15 % of its cycles busy there).
-struct FDiv {
+// m = 1, and umulhi(n, 1) = 0 leaves n >> s.
+struct FDivB {
   unsigned d, m, s;
-  __device__ __forceinline__ explicit FDiv(unsigned d_) : d(d_) {
+  __device__ __forceinline__ unsigned div(unsigned n) const {
+    return (__umulhi(n, m) + n) >> s;
+  }
+};
+// Divisors that are launch constants, built once per kernel: the 64-bit
+// division stays on the uniform path, and so do m and s (built as below they
+// took 6 more registers a thread, and the strided fixed-point FWHT spilled).
+struct FDiv : FDivB {
+  __device__ __forceinline__ explicit FDiv(unsigned d_) {
+    d = d_;
+    s = d > 1 ? 32 - __clz(d - 1) : 0;  // ceil(log2 d)
+    m = (d & (d - 1)) == 0
+            ? 1u
+            : (unsigned)(((1ull << 32) * ((1ull << s) - d)) / d + 1);
+  }
+};
+// Divisors built per stage or per tile: the quotient of m is estimated in
+// float (within 2^10) and corrected by its remainder, since a 64-bit division
+// in every thread takes the FP64 pipe, the slowest of this GPU (Fourier(6000)
+// x 64: 15 % of its cycles busy there; 30.8 -> 28.7 us without).
+struct FDivF : FDivB {
+  __device__ __forceinline__ explicit FDivF(unsigned d_) {
+    d = d_;
     s = d > 1 ? 32 - __clz(d - 1) : 0;  // ceil(log2 d)
     m = 1u;
     if (d & (d - 1)) {
@@ -380,9 +399,6 @@ struct FDiv {
       if (rem >= (i64)d) ++q;
       m = q + 1u;
     }
-  }
-  __device__ __forceinline__ unsigned div(unsigned n) const {
-    return (__umulhi(n, m) + n) >> s;
   }
 };
 
@@ -523,7 +539,7 @@ __device__ __forceinline__ void fft_stage_body(C *sm, int Lp, int B, int Lf,
   const int M = Mprev / R;
   const int nw = Lf / R;
   const int total = B * nw;
-  const FDiv dnw((unsigned)nw), dM((unsigned)M);
+  const FDivF dnw((unsigned)nw), dM((unsigned)M);
   const int lgB = __ffs(B) - 1;
   const int tscale = (Mprev & (Mprev - 1)) == 0 ? Lf >> (__ffs(Mprev) - 1)
                                                  : Lf / Mprev;
@@ -1073,8 +1089,8 @@ __host__ __device__ __forceinline__ size_t launch_smem(int B, int Lp, int esz,
 
 // per-vector addressing of tile `tile` (vector indices below 2^31)
 __device__ __forceinline__ void setup_tile(const Step &p, VInfo *vi,
-                                           i64 tile, const FDiv &dV,
-                                           const FDiv &dci, const FDiv &dco,
+                                           i64 tile, const FDivB &dV,
+                                           const FDivB &dci, const FDivB &dco,
                                            i64 nvec, int tid, int T) {
   for (int b = tid; b < p.B; b += T) {
     const i64 gv = tile * p.B + b;
@@ -1140,7 +1156,7 @@ __device__ __forceinline__ void tma_issue_store(const Step &p, const E *sm,
 // padded layout (each chunk is contiguous and 16-byte aligned there).
 template <class E, int LAY>
 __device__ __forceinline__ void issue_load(const Step &p, E *sm, unsigned bar,
-                                           i64 tile, const FDiv &dV, i64 nvec,
+                                           i64 tile, const FDivB &dV, i64 nvec,
                                            int tid, int T) {
   if constexpr (LAY == 1) {
     if (tid == 0) tma_issue_load<E>(p, sm, bar, tile);
@@ -1186,7 +1202,7 @@ __device__ __forceinline__ void issue_load(const Step &p, E *sm, unsigned bar,
 
 template <class E, int LAY>
 __device__ __forceinline__ void issue_store(const Step &p, const E *sm,
-                                            i64 tile, const FDiv &dV,
+                                            i64 tile, const FDivB &dV,
                                             i64 nvec, int tid, int T) {
   if constexpr (LAY == 1) {
     if (tid == 0) tma_issue_store<E>(p, sm, tile);
