@@ -863,7 +863,9 @@ __device__ __forceinline__ void d2hl(double d, unsigned sub, int thr,
 // (h + l) 2^s as a float64, rounded to nearest: h's bits widened exactly, l
 // converted to units in the last place of that float64 and added to its bit
 // pattern (an integer addition: carries move into the exponent as they
-// should).  bias = (s + 896) << 20; s plain (df_scale_plain).
+// should).  bias = (s + 896) << 20; s plain (df_scale_plain).  A head that is
+// Inf or NaN (from the operator's data or an overflow; its tail is NaN after
+// the renormalisation, so n = 0) stays Inf or NaN.
 __device__ __forceinline__ double hl2d(float h, float l, int bias) {
   const unsigned u = (unsigned)__float_as_int(h);
   const unsigned eb = u & 0x7F800000u;
@@ -874,7 +876,8 @@ __device__ __forceinline__ double hl2d(float h, float l, int bias) {
   int n = __float2int_rn((l * 16777216.f) * w);
   // below a power of two the spacing halves
   if ((u & 0x007FFFFFu) == 0u && n < 0) n += n;
-  const unsigned hi = ((unsigned)((int)u >> 3) & 0x8FFFFFFFu) + (unsigned)bias;
+  unsigned hi = ((unsigned)((int)u >> 3) & 0x8FFFFFFFu) + (unsigned)bias;
+  if (eb == 0x7F800000u) hi |= 0x7FF00000u;
   const unsigned lo = u << 29;
   i64 b = (i64)(((unsigned long long)hi << 32) | lo) + (i64)n;
   if (eb == 0u) b = 0;

@@ -1,0 +1,88 @@
+"""The double-float register kernels (register convolution, long-vector FFT
+and convolution) where the operator, not the input, leaves the ordinary
+range: NaN and Inf in an operator's own data, results that overflow, very
+small results, and elements far below their vector's largest.  References
+in float64 numpy."""
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip('torch')
+pytestmark = pytest.mark.gpu
+
+
+def _cplx(rng, *shape):
+    return rng.standard_normal(shape) + 1j * rng.standard_normal(shape)
+
+
+def _conv(c, x):
+    return np.fft.ifft(np.fft.fft(c)[:, None] * np.fft.fft(x, axis=0), axis=0)
+
+
+def _forward(op, x):
+    t = torch.from_numpy(np.ascontiguousarray(x.T)).cuda().t()
+    y = op.forward(t)
+    op.check()
+    return y.cpu().numpy()
+
+
+# rconv: one warp a vector; rxconv: whole columns; rxfft: the outer passes of
+# long columns
+ROUTES = [(16, 'rconv'), (128, 'rconv'), (512, 'rxconv'), (4096, 'rxconv'),
+          (1 << 14, 'rxfft'), (1 << 17, 'rxfft')]
+
+
+def _routed(op, route, direction=0):
+    assert route in op.plan(np.complex128).describe(direction)
+    return op
+
+
+@pytest.mark.parametrize('bad', [np.nan, np.inf])
+@pytest.mark.parametrize('n,route', ROUTES)
+def test_non_finite_filter(n, route, bad):
+    import fastmat_gb300 as fm
+    rng = np.random.default_rng(n)
+    c = _cplx(rng, n)
+    c[3] = bad
+    y = _forward(_routed(fm.Circulant(c), route), _cplx(rng, n, 2))
+    assert not np.isfinite(y).any()
+
+
+@pytest.mark.parametrize('bad', [np.nan, np.inf])
+@pytest.mark.parametrize('n,route', ROUTES)
+def test_non_finite_product_of_the_storer(n, route, bad):
+    import fastmat_gb300 as fm
+    rng = np.random.default_rng(n)
+    c, d, x = _cplx(rng, n), _cplx(rng, n), _cplx(rng, n, 2)
+    d[5] = bad
+    y = _forward(_routed(fm.Product(fm.Diag(d), fm.Circulant(c)), route), x)
+    assert not np.isfinite(y[5]).any()
+    keep = np.arange(n) != 5
+    r = d[keep, None] * _conv(c, x)[keep]
+    assert np.abs(y[keep] - r).max() <= 1e-12 * np.abs(r).max()
+
+
+@pytest.mark.parametrize('bad', [np.nan, np.inf])
+@pytest.mark.parametrize('n,route', ROUTES)
+def test_non_finite_product_of_the_loader(n, route, bad):
+    import fastmat_gb300 as fm
+    rng = np.random.default_rng(n)
+    d = _cplx(rng, n)
+    d[5] = bad
+    op = fm.Product(fm.Circulant(_cplx(rng, n)), fm.Diag(d))
+    y = _forward(_routed(op, route), _cplx(rng, n, 2))
+    assert not np.isfinite(y).any()
+
+
+@pytest.mark.parametrize('n,route', ROUTES)
+def test_overflow_is_not_finite(n, route):
+    """Results beyond the arithmetic's range (2^128 of the largest input) are
+    Inf or NaN, never a wrong number."""
+    import fastmat_gb300 as fm
+    rng = np.random.default_rng(n)
+    c, d, x = _cplx(rng, n), _cplx(rng, n), _cplx(rng, n, 2)
+    op = fm.Product(fm.Diag(d * 1e25), fm.Circulant(c * 1e25))
+    y = _forward(_routed(op, route), x)
+    r = 1e50 * (d[:, None] * _conv(c, x))
+    bad = np.abs(y - r) > 1e-12 * np.abs(r).max()
+    assert not (bad & np.isfinite(y.real) & np.isfinite(y.imag)).any()
