@@ -864,16 +864,16 @@ __device__ __forceinline__ void d2hl(double d, unsigned sub, int thr,
 // converted to units in the last place of that float64 and added to its bit
 // pattern (an integer addition: carries move into the exponent as they
 // should).  bias = (s + 896) << 20; s plain (df_scale_plain).  A head that is
-// Inf or NaN (from the operator's data or an overflow; its tail is NaN after
-// the renormalisation, so n = 0) stays Inf or NaN.
+// Inf or NaN (from the operator's data or an overflow) stays Inf or NaN.
 __device__ __forceinline__ double hl2d(float h, float l, int bias) {
   const unsigned u = (unsigned)__float_as_int(h);
   const unsigned eb = u & 0x7F800000u;
-  // +-2^(52 - e) in two factors (either alone could leave float's range):
-  // one unit of the result's last place is 2^(e - 52)
+  // +-2^(52 - e) in two factors: one unit of the result's last place is
+  // 2^(e - 52).  The first is a normal float for every normal h and brings
+  // every l, subnormal ones too, to 2^-23 or less (0 for Inf and NaN: n = 0).
   const float w =
-      __int_as_float((int)(((282u << 23) - eb) | (u & 0x80000000u)));
-  int n = __float2int_rn((l * 16777216.f) * w);
+      __int_as_float((int)(((255u << 23) - eb) | (u & 0x80000000u)));
+  int n = __float2int_rn((l * w) * 2251799813685248.f);
   // below a power of two the spacing halves
   if ((u & 0x007FFFFFu) == 0u && n < 0) n += n;
   unsigned hi = ((unsigned)((int)u >> 3) & 0x8FFFFFFFu) + (unsigned)bias;

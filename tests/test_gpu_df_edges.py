@@ -86,3 +86,27 @@ def test_overflow_is_not_finite(n, route):
     r = 1e50 * (d[:, None] * _conv(c, x))
     bad = np.abs(y - r) > 1e-12 * np.abs(r).max()
     assert not (bad & np.isfinite(y.real) & np.isfinite(y.imag)).any()
+
+
+@pytest.mark.parametrize('e', range(-120, -99, 2))
+@pytest.mark.parametrize('n,route', ROUTES)
+def test_small_results_keep_their_tails(n, route, e):
+    """Results of 2^e of the vector's largest element, by two factors of
+    2^(e / 2): what float's subnormals hold of the tails is stored."""
+    import fastmat_gb300 as fm
+    rng = np.random.default_rng(n)
+    c, d, x = _cplx(rng, n), _cplx(rng, n), _cplx(rng, n, 3)
+    f = 2.0 ** (e // 2)
+    C, D = fm.Circulant(c * f), fm.Diag(d * f)
+    if route == 'rconv':
+        # (its storer converts vectors with a product of its own as other
+        # kernels do, which drops subnormal tails)
+        op, r, terms = fm.Product(C, D), _conv(c, d[:, None] * x), n
+    else:
+        op, r, terms = fm.Product(D, C), d[:, None] * _conv(c, x), 1
+    y = _forward(_routed(op, route), x)
+    y = np.ldexp(y.real, -e) + 1j * np.ldexp(y.imag, -e)
+    # the engine's 1e-12, and the tails of the products of that size, some
+    # 10 roundings to multiples of 2^-149 of the column's largest element
+    tails = np.ldexp(np.abs(x).max() * terms, -145 - e)
+    assert np.abs(y - r).max() <= 1e-12 * np.abs(r).max() + tails
