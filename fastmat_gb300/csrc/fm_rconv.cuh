@@ -301,11 +301,11 @@ template <int P>
 __device__ __forceinline__ void rx_in(dfq (&x)[P], const double2 (&d)[P],
                                       int s) {
   const unsigned sub = (unsigned)(s + 896) << 23;
-  const int thr = max(s + 896 + 53, 1) << 20;
+  const int thr = max(s + 896 + 1, 1) << 20, thl = max(s + 896 + 53, 1) << 20;
 #pragma unroll
   for (int r = 0; r < P; ++r) {
-    d2hl(d[r].x, sub, thr, x[r].h.x, x[r].l.x);
-    d2hl(d[r].y, sub, thr, x[r].h.y, x[r].l.y);
+    d2hl(d[r].x, sub, thr, thl, x[r].h.x, x[r].l.x);
+    d2hl(d[r].y, sub, thr, thl, x[r].h.y, x[r].l.y);
   }
 }
 template <int P, class E, class F>

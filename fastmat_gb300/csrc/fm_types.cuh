@@ -825,18 +825,15 @@ __device__ __forceinline__ void store_elem(void *p, int type, i64 idx, E v,
 }
 
 // ---- float64 <-> packed double-float in the register kernels.  A vector
-// is scaled by 2^-s, s = its largest exponent minus kDfTop, so its largest
-// element sits at 2^kDfTop; elements more than 2^(74 + kDfTop) below it
-// (2^-84, far below the 2^-48 of the arithmetic) flush to zero.  kDfTop
-// leaves the operator's own magnitude most of float's exponent range on
-// both sides (results 2^-109 .. 2^117 of the largest element keep their
-// tails).
+// is scaled by 2^-s, s = its largest exponent minus the bias, so its largest
+// element sits at 2^0 .. 2^1 and results up to 2^127 of it fit; elements more
+// than 2^126 below it flush to zero, the tails of those more than 2^74 below
+// it (as the tile conversions, d2df_scaled).
 // A vector holding Inf or NaN gets the s that maps the exponent field of
 // Inf / NaN to float's, so those elements stay Inf / NaN.
-constexpr int kDfTop = 10;
 // largest (hi & 0x7fffffff) of a vector's words -> s
 __device__ __forceinline__ int df_scale(int emax) {
-  return emax >= 0x7FF ? 896 : emax - 1023 - kDfTop;
+  return emax >= 0x7FF ? 896 : emax - 1023;
 }
 // s for which no result can leave the float64 range (results lie within
 // 2^-127 .. 2^127 of 2^s)
@@ -844,9 +841,9 @@ __device__ __forceinline__ bool df_scale_plain(int s) {
   return s >= -890 && s <= 890;
 }
 // d 2^-s as h + l: h the leading 24 significand bits (truncated), l the
-// other 29 rounded to a float.  sub = (s + 896) << 23, thr = the smallest
-// high word (sign cleared) that does not flush.
-__device__ __forceinline__ void d2hl(double d, unsigned sub, int thr,
+// other 29 rounded to a float.  sub = (s + 896) << 23; thr, thl = the
+// smallest high words (sign cleared) whose head and whose tail do not flush.
+__device__ __forceinline__ void d2hl(double d, unsigned sub, int thr, int thl,
                                      float &h, float &l) {
   const unsigned hi = (unsigned)__double2hiint(d),
                  lo = (unsigned)__double2loint(d);
@@ -856,9 +853,9 @@ __device__ __forceinline__ void d2hl(double d, unsigned sub, int thr,
   // the remaining bits weigh 2^(ef - 127 - 52) each
   const float f = __int_as_float((int)((t & 0x7F800000u) - (52u << 23)));
   const float r = (float)(lo & 0x1FFFFFFFu) * f;
-  const bool keep = (int)(hi & 0x7FFFFFFFu) >= thr;
-  h = keep ? __int_as_float((int)(t | sg)) : 0.f;
-  l = keep ? __int_as_float((int)(__float_as_int(r) | sg)) : 0.f;
+  const int mag = (int)(hi & 0x7FFFFFFFu);
+  h = mag >= thr ? __int_as_float((int)(t | sg)) : 0.f;
+  l = mag >= thl ? __int_as_float((int)(__float_as_int(r) | sg)) : 0.f;
 }
 // (h + l) 2^s as a float64, rounded to nearest: h's bits widened exactly, l
 // converted to units in the last place of that float64 and added to its bit

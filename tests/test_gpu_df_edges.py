@@ -107,6 +107,45 @@ def test_small_results_keep_their_tails(n, route, e):
     y = _forward(_routed(op, route), x)
     y = np.ldexp(y.real, -e) + 1j * np.ldexp(y.imag, -e)
     # the engine's 1e-12, and the tails of the products of that size, some
-    # 10 roundings to multiples of 2^-149 of the column's largest element
-    tails = np.ldexp(np.abs(x).max() * terms, -145 - e)
-    assert np.abs(y - r).max() <= 1e-12 * np.abs(r).max() + tails
+    # 10 roundings to multiples of 2^-149 of the column's largest element;
+    # real and imaginary parts below 2^-126 of that element flush to zero
+    top = np.abs(x).max()
+    tails = np.ldexp(top * terms, -145 - e)
+    gone = np.ldexp(top, -125 - e)
+    for u, v in ((y.real, r.real), (y.imag, r.imag)):
+        err = np.where((u == 0) & (np.abs(v) <= gone), 0.0, np.abs(u - v))
+        assert err.max() <= 1e-12 * np.abs(r).max() + tails
+
+
+@pytest.mark.parametrize('n,route', ROUTES[:3])
+def test_results_up_to_the_range_of_float(n, route):
+    """Results near 2^124 of the vector's largest element."""
+    import fastmat_gb300 as fm
+    rng = np.random.default_rng(n)
+    c, x = np.zeros(n, dtype=np.complex128), _cplx(rng, n, 3)
+    c[:2] = [1.0, 0.5j]
+    x /= np.abs(x).max()
+    # (2^121: the transform of x stays below 2^6.5 at 512 points, and the
+    # spectrum's 1 / n returns what the sums of the inverse take)
+    y = _forward(_routed(fm.Circulant(np.ldexp(c.real, 121) +
+                                      1j * np.ldexp(c.imag, 121)), route), x)
+    y = np.ldexp(y.real, -121) + 1j * np.ldexp(y.imag, -121)
+    r = _conv(c, x)
+    assert np.abs(y - r).max() <= 1e-12 * np.abs(r).max()
+
+
+@pytest.mark.parametrize('n,route', ROUTES)
+def test_elements_far_below_the_largest_keep_their_heads(n, route):
+    """A Diag on the loader that removes the largest element: the others,
+    2^-100 of it, keep the 24 bits of their heads."""
+    import fastmat_gb300 as fm
+    rng = np.random.default_rng(n)
+    c, d, x = _cplx(rng, n), np.full(n, 2.0 ** 80, complex), _cplx(rng, n, 2)
+    x = np.ldexp(x.real, -100) + 1j * np.ldexp(x.imag, -100)
+    x[7] = 1.0
+    d[7] = 0.0
+    y = _forward(_routed(fm.Product(fm.Circulant(c), fm.Diag(d)), route), x)
+    r = _conv(c, d[:, None] * x)
+    # heads truncated to 24 bits: 2^-23 of each element, and at most
+    # sum |c| / |y| ~ 1 / sqrt(n) .. 1 of that in the result
+    assert np.abs(y - r).max() <= 2.0 ** -22 * np.abs(r).max()
