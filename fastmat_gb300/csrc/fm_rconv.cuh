@@ -297,15 +297,22 @@ __device__ __forceinline__ int rx_max(const double2 (&d)[P]) {
   for (int r = 0; r < P; ++r) e = max(e, max(raw_hi(d[r].x), raw_hi(d[r].y)));
   return e;
 }
-template <int P>
+template <bool RN, int P>
 __device__ __forceinline__ void rx_in(dfq (&x)[P], const double2 (&d)[P],
                                       int s) {
-  const unsigned sub = (unsigned)(s + 896) << 23;
-  const int thr = max(s + 896 + 1, 1) << 20, thl = max(s + 896 + 53, 1) << 20;
+  const int base = s + 896;
+  const int thr = max(base + 1, 1) << 20, thl = max(base + 53, 1) << 20;
 #pragma unroll
   for (int r = 0; r < P; ++r) {
-    d2hl(d[r].x, sub, thr, thl, x[r].h.x, x[r].l.x);
-    d2hl(d[r].y, sub, thr, thl, x[r].h.y, x[r].l.y);
+    d2hl<RN>(d[r].x, base, thr, thl, x[r].h.x, x[r].l.x);
+    d2hl<RN>(d[r].y, base, thr, thl, x[r].h.y, x[r].l.y);
+  }
+  if (RN && s == kDfNonFinite) {
+#pragma unroll
+    for (int r = 0; r < P; ++r) {
+      if (raw_hi(d[r].x) >= 0x7FF00000) x[r].h.x = __int_as_float(0x7FFFFFFF);
+      if (raw_hi(d[r].y) >= 0x7FF00000) x[r].h.y = __int_as_float(0x7FFFFFFF);
+    }
   }
 }
 template <int P, class E, class F>
@@ -489,8 +496,8 @@ __global__ void __launch_bounds__(FM_RC_THREADS, (RcOcc<E, L>::v))
 #pragma unroll
       for (int o = G / 2; o >= 1; o /= 2)
         emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o, G));
-      sexp = df_scale(emax >> 20);
-      rx_in<P>(x, d, sexp);
+      sexp = df_scale<false>(emax >> 20);
+      rx_in<false>(x, d, sexp);
     } else {
 #pragma unroll
       for (int r = 0; r < P; ++r) x[r] = d[r];

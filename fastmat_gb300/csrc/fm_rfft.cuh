@@ -398,8 +398,8 @@ __global__ void __launch_bounds__(RxShape<E, L>::TF,
       __syncthreads();
       if (emax > 0) atomicMax(sexp + lane, emax);
       __syncthreads();
-      s = df_scale(sexp[lane] >> 20);
-      rx_in<P>(x, d, s);
+      s = df_scale<true>(sexp[lane] >> 20);
+      rx_in<true>(x, d, s);
     } else {
 #pragma unroll
       for (int r = 0; r < P; ++r) x[r] = E{d[r].x, d[r].y};
@@ -481,8 +481,8 @@ __global__ void __launch_bounds__(RxShape<E, L>::TC,
         __syncthreads();
         emax = sexp[q];
       }
-      s = df_scale(emax >> 20);
-      rx_in<P>(x, d, s);
+      s = df_scale<true>(emax >> 20);
+      rx_in<true>(x, d, s);
     } else {
 #pragma unroll
       for (int r = 0; r < P; ++r) x[r] = E{d[r].x, d[r].y};

@@ -133,8 +133,8 @@ __global__ void __launch_bounds__(RsfShape<E, L>::T, (RsfOcc<E>::v))
       __syncthreads();
       if (emax > 0) atomicMax(sexp + v, emax);
       __syncthreads();
-      s = df_scale(sexp[v] >> 20);
-      rx_in<P>(x, d, s);
+      s = df_scale<false>(sexp[v] >> 20);
+      rx_in<false>(x, d, s);
     } else {
 #pragma unroll
       for (int r = 0; r < P; ++r) x[r] = E{d[r].x, d[r].y};

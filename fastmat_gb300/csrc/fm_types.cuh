@@ -834,33 +834,55 @@ __device__ __forceinline__ void store_elem(void *p, int type, i64 idx, E v,
 // element sits at 2^0 .. 2^1 and results up to 2^127 of it fit; elements more
 // than 2^126 below it flush to zero, the tails of those more than 2^74 below
 // it (as the tile conversions, d2df_scaled).
-// A vector holding Inf or NaN gets the s that maps the exponent field of
-// Inf / NaN to float's, so those elements stay Inf / NaN.
-// largest (hi & 0x7fffffff) of a vector's words -> s
-__device__ __forceinline__ int df_scale(int emax) {
-  return emax >= 0x7FF ? 896 : emax - 1023;
+// A vector holding Inf or NaN: with truncated heads s = 896 maps the exponent
+// field of Inf / NaN to float's, so those elements stay Inf / NaN; with rounded
+// ones (a carry would leave that field) s = kDfNonFinite, and those elements
+// enter the transform as NaN (rx_in).
+constexpr int kDfNonFinite = 0x7FF - 1023;
+// largest (hi & 0x7fffffff) of a vector's words >> 20 -> s
+template <bool RN> __device__ __forceinline__ int df_scale(int emax) {
+  return !RN && emax >= 0x7FF ? 896 : emax - 1023;
 }
 // s for which no result can leave the float64 range (results lie within
 // 2^-127 .. 2^127 of 2^s)
 __device__ __forceinline__ bool df_scale_plain(int s) {
   return s >= -890 && s <= 890;
 }
-// d 2^-s as h + l: h the leading 24 significand bits (truncated), l the
-// other 29 rounded to a float.  sub = (s + 896) << 23; thr, thl = the
-// smallest high words (sign cleared) whose head and whose tail do not flush.
-__device__ __forceinline__ void d2hl(double d, unsigned sub, int thr, int thl,
+// d 2^-s as h + l.  RN (finite d): h is d rounded to 24 significand bits
+// (halves away from zero), l the remainder, at most 2^28 units of d's last
+// place, rounded to a float: h + l is within 2^-49 |d|.  Otherwise h is
+// truncated, l the other 29 bits, h + l within 2^-48 |d|, with fewer
+// operations.  The long-vector transforms take RN, as their loads of
+// gathered and converted elements (d2df) always did (Toeplitz(3000, 5001) on
+// real data: 1.02e-14 from 64 bits, truncated 1.18e-14; chain adjoint 2^18 x
+// 32 491 us, truncated 484); in the Kron modes' kernels, whose loads always
+// truncated, it would cost 3 % of the FP64 form (2147 -> 2211 us).
+// base = s + 896; thr, thl = the smallest high words (sign cleared) whose
+// head and whose tail do not flush.
+template <bool RN>
+__device__ __forceinline__ void d2hl(double d, int base, int thr, int thl,
                                      float &h, float &l) {
   const unsigned hi = (unsigned)__double2hiint(d),
                  lo = (unsigned)__double2loint(d);
   const unsigned sg = hi & 0x80000000u;
-  // exponent field (9 bits) and 23 significand bits, exponent rebased
-  const unsigned t = __funnelshift_l(lo, hi, 3) - sub;
-  // the remaining bits weigh 2^(ef - 127 - 52) each
-  const float f = __int_as_float((int)((t & 0x7F800000u) - (52u << 23)));
-  const float r = (float)(lo & 0x1FFFFFFFu) * f;
+  unsigned t;  // exponent field, rebased, and 23 significand bits
+  float r;     // the remainder: its units are 2^(ef - 127 - 52)
+  if constexpr (RN) {
+    // the next bit is rounded in; a carry moves into the exponent as it
+    // should and leaves a negative remainder (ef: the field before it)
+    t = (__funnelshift_l(lo, hi, 4) - (((unsigned)base << 24) - 1u)) >> 1;
+    const unsigned f =
+        (((hi << 3) - ((unsigned)(base + 52) << 23)) & 0x7F800000u) | sg;
+    r = (float)((int)(lo << 3) >> 3) * __int_as_float((int)f);
+  } else {
+    t = __funnelshift_l(lo, hi, 3) - ((unsigned)base << 23);
+    r = (float)(lo & 0x1FFFFFFFu) *
+        __int_as_float((int)((t & 0x7F800000u) - (52u << 23)));
+    r = __int_as_float(__float_as_int(r) | (int)sg);
+  }
   const int mag = (int)(hi & 0x7FFFFFFFu);
   h = mag >= thr ? __int_as_float((int)(t | sg)) : 0.f;
-  l = mag >= thl ? __int_as_float((int)(__float_as_int(r) | sg)) : 0.f;
+  l = mag >= thl ? r : 0.f;
 }
 // (h + l) 2^s as a float64, rounded to nearest: h's bits widened exactly, l
 // converted to units in the last place of that float64 and added to its bit

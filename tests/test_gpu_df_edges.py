@@ -173,3 +173,43 @@ def test_products_round_like_normalised_double_floats():
     # float32: 0.666 2^-48 with normalised products, 0.743 with products
     # renormalised once after their sum; the bound lies between
     assert np.sqrt(np.mean(np.square(err))) <= 0.70 * 2.0 ** -48
+
+
+@pytest.mark.parametrize('real', [False, True])
+@pytest.mark.parametrize('n,route', [(512, 'rxconv'), (4096, 'rxconv'),
+                                     (1 << 17, 'rxfft')])
+def test_inputs_keep_49_bits(n, route, real):
+    """A one-hot column through the identity filter: every operation of the
+    transforms is exact (sums of equal values, products with 1 and powers of
+    two), what remains is the conversion of the input, heads rounded to 24
+    bits and tails to 24 of 29."""
+    import fastmat_gb300 as fm
+    rng = np.random.default_rng(n)
+    m = 2048 if n <= 4096 else 128
+    c = np.zeros(n, dtype=np.complex128)
+    c[0] = 1.0
+    x = np.zeros((n, m), dtype=np.float64 if real else np.complex128)
+    x[0] = rng.standard_normal(m) if real else _cplx(rng, m)
+    y = _forward(_routed(fm.Circulant(c), route), x)
+    assert (np.abs(y[0].real - x[0].real) <=
+            2.0 ** -49 * np.abs(x[0].real)).all()
+    if not real:
+        # (a part below the vector's largest flushes no bits here: 2^-74)
+        assert (np.abs(y[0].imag - x[0].imag) <=
+                2.0 ** -49 * np.abs(x[0].imag)).all()
+    assert not y[1:].any()
+
+
+@pytest.mark.parametrize('n,route', ROUTES)
+def test_nan_payloads(n, route):
+    """NaN of any payload (all ones: a carry of the rounding) stays NaN."""
+    import fastmat_gb300 as fm
+    rng = np.random.default_rng(n)
+    x = _cplx(rng, n, 2)
+    x.view(np.float64).view(np.uint64).reshape(n, 2, 2)[1, 0, 1] = (
+        0x7FFFFFFFFFFFFFFF)
+    c = _cplx(rng, n)
+    y = _forward(_routed(fm.Circulant(c), route), x)
+    assert not np.isfinite(y[:, 0]).any()
+    r = _conv(c, x[:, 1:])
+    assert np.abs(y[:, 1:] - r).max() <= 1e-12 * np.abs(r).max()
