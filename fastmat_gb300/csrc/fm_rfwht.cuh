@@ -96,6 +96,11 @@ __device__ __forceinline__ int rf_pos(int h, int s, int r, int w) {
   return ((h >> s) << (s + w)) | (r << s) | (h & ((1 << s) - 1));
 }
 
+// levels of the first pass
+template <class E, int L> __host__ __device__ constexpr int rf_w0() {
+  return rf_log2(L) < RfLane<E>::PB ? rf_log2(L) : RfLane<E>::PB;
+}
+
 // largest exponent word of a thread's points
 template <int P>
 __device__ __forceinline__ int rf_max(const double (&d)[P]) {
@@ -168,13 +173,18 @@ template <class E, int L, int S0>
 __device__ __forceinline__ void rf_pass(E (&x)[RfLane<E>::P]) {
   constexpr int P = RfLane<E>::P, PB = RfLane<E>::PB, K = rf_log2(L);
   constexpr int W = K - S0 < PB ? K - S0 : PB;
-  typedef typename Lazy<E>::type LE;
-  LE v[P];
+  constexpr int WN = K - S0 - W < PB ? K - S0 - W : PB;  // next pass (0: none)
+  if constexpr (RfLane<E>::fixed && WN > 0) {
+    // make room for the next pass, rounded: half a unit on a group's first
+    // point is half a unit on each of its results
 #pragma unroll
-  for (int j = 0; j < P; ++j) v[j] = to_lazy(x[j]);
-  rf_levels<LE, P, W>(v);
+    for (int u = 0; u < (P >> W); ++u) x[u << W].v += 1ll << (WN - 1);
+  }
+  rf_levels<E, P, W>(x);
+  if constexpr (RfLane<E>::fixed && WN > 0) {
 #pragma unroll
-  for (int j = 0; j < P; ++j) x[j] = from_lazy(v[j]);
+    for (int j = 0; j < P; ++j) x[j].v >>= WN;
+  }
 }
 
 // registers laid out for the pass at bit offset SA -> exchange buffer ->
@@ -248,7 +258,7 @@ __device__ __forceinline__ void rf_finish(
     __syncthreads();
     emax = sexp[vl] >> 20;
 #pragma unroll
-    for (int r = 0; r < P; ++r) x[r] = d2fx(d[r], emax, rf_log2(L));
+    for (int r = 0; r < P; ++r) x[r] = d2fx(d[r], emax, rf_w0<E, L>());
   } else {
 #pragma unroll
     for (int r = 0; r < P; ++r) x[r] = d[r];
@@ -396,7 +406,7 @@ __device__ __forceinline__ void rs_batch(const RfStep &p, i64 bt, E *xb,
     __syncthreads();
     emax = sexp[v] >> 20;
 #pragma unroll
-    for (int r = 0; r < P; ++r) x[r] = d2fx(d[r], emax, rf_log2(L));
+    for (int r = 0; r < P; ++r) x[r] = d2fx(d[r], emax, rf_w0<E, L>());
   } else {
 #pragma unroll
     for (int r = 0; r < P; ++r) x[r] = d[r];

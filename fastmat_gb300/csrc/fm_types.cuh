@@ -908,36 +908,45 @@ __device__ __forceinline__ double hl2d(float h, float l, int bias) {
   return __longlong_as_double(b);
 }
 // ---- 64-bit fixed point for the register FWHT of float64 data: sums and
-// differences only, so a vector of 2^K points scaled to below 2^(63 - K)
-// adds without rounding (an addition is 2 integer instructions where an
+// differences only, so points scaled to below 2^(63 - W) take W levels
+// without rounding (an addition is 2 integer instructions where an
 // unnormalised double-float one is 8, and they issue at the same rate:
-// measured 64 int64 additions per clock and SM).  The only errors are the
-// scaling's truncation, at most 2^(K - 62) of the vector's largest element
-// (2^-50 at 4096 points; none for elements near the largest up to 1024
-// points), and the final rounding.
+// measured 64 int64 additions per clock and SM).  Only the W levels of a
+// pass are provided for: the points are rounded to nearest when they are
+// converted and again, W bits down, between two passes (rf_pass).  A result
+// is off by at most half a unit of each rounding, summed over the points the
+// levels after it add up: 3 2^-48 of the vector's largest element at 4096
+// points if every rounding agrees (6e-17 of the largest result measured on
+// random data), and the final rounding.  (Providing for all K levels at the
+// conversion, as sums without any rounding would need, leaves 2^(K - 62) of
+// the largest element for each of 2^K points of one sign: one element of 1 on
+// a background of 1e-6 then came out 2e-12 off.)
 struct fx {
   i64 v;
 };
 __device__ __forceinline__ fx addv(fx a, fx b) { return fx{a.v + b.v}; }
 __device__ __forceinline__ fx subv(fx a, fx b) { return fx{a.v - b.v}; }
-// d as fixed point: emax the largest exponent field of the vector
-__device__ __forceinline__ fx d2fx(double d, int emax, int K) {
+// d as fixed point: emax the largest exponent field of the vector, W the
+// levels of the first pass
+__device__ __forceinline__ fx d2fx(double d, int emax, int W) {
   const unsigned hi = (unsigned)__double2hiint(d),
                  lo = (unsigned)__double2loint(d);
   const int ex = (int)((hi >> 20) & 0x7FFu);
   // significand with its leading bit at bit 63, then down to weight
-  // 2^(63 - K) for the largest exponent; zeros and subnormals vanish
+  // 2^(63 - W) for the largest exponent, the last bit shifted out rounded in;
+  // zeros and subnormals vanish
   const unsigned mh = __funnelshift_l(lo, hi, 11) | 0x80000000u;
   const unsigned long long u =
       ((unsigned long long)mh << 32) | (unsigned)(lo << 11);
-  const unsigned n = ex ? (unsigned)(emax - ex + K + 1) : 64u;
+  const unsigned n = ex ? (unsigned)(emax - ex + W) : 64u;
   unsigned long long w;  // (a shift by 64 or more gives 0)
   asm("shr.u64 %0, %1, %2;" : "=l"(w) : "l"(u), "r"(n));
   const i64 s = (i64)((int)hi >> 31);
-  return fx{((i64)w ^ s) - s};
+  return fx{(((i64)w ^ s) + (i64)(1u + (hi >> 31))) >> 1};
 }
-// fixed point to float64, rounded to nearest; plain: no result can leave
-// the float64 range (emax between 80 and 2020), nan: ORed into the high word
+// fixed point to float64 after K levels, rounded to nearest; plain: no
+// result can leave the float64 range (emax between 80 and 2020), nan: ORed
+// into the high word
 __device__ __forceinline__ double fx2d(fx a, int emax, int K, bool plain,
                                        unsigned nan) {
   const i64 s = a.v >> 63;
