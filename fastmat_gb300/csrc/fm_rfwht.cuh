@@ -82,7 +82,7 @@ template <class E, int L>
 __host__ __device__ constexpr size_t rf_smem() {
   typedef RfShape<E, L> S;
   return (size_t)S::VPC * S::Ls * sizeof(typename S::Raw) +
-         (size_t)S::VPC * S::Lx * sizeof(E) + 64;
+         (size_t)S::VPC * S::Lx * sizeof(E) + 2 * S::VPC * sizeof(int);
 }
 template <class E, int L> struct RfOcc {
   static constexpr int v = RfShape<E, L>::T > 256 ? 1 : 2;
@@ -109,23 +109,49 @@ __device__ __forceinline__ int rf_max(const double (&d)[P]) {
   for (int r = 0; r < P; ++r) e = max(e, raw_hi(d[r]));
   return e;
 }
-// registers to raw words (emax: the vector's largest exponent field; a
-// vector holding Inf or NaN gives NaN throughout, as its sums do)
+// Vectors that go to double-float instead of fixed point: those with Inf or
+// NaN, and those where the points of some thread, 16 neighbours, all lie more
+// than 2^11 below the largest (mx, mn: the vector's largest and smallest
+// non-zero maximum of a thread's points).  Fixed point keeps every element to
+// 2^-60 of the largest, 48 bits of those down to 2^-11; where whole groups are
+// smaller, the large elements may cancel in some results, which then hang on
+// the small ones' own bits.  Random data never gets here (a group of 16
+// normal variates: 2^-150); the double-float form of Hadamard(18) x 48 takes
+// about twice the time.
+__device__ __forceinline__ bool rf_wide(int mx, int mn) {
+  return mx >= 0x7FF00000 || (mn >> 20) + 11 < (mx >> 20);
+}
+// largest and smallest of a vector's mx, mn over its WV lanes
+template <int WV> __device__ __forceinline__ void rf_reduce(int &mx, int &mn) {
+  if constexpr (WV == 32) {
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    mn = __reduce_min_sync(0xffffffffu, mn);
+  } else {
+#pragma unroll
+    for (int o = WV / 2; o >= 1; o /= 2) {
+      mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o, WV));
+      mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o, WV));
+    }
+  }
+}
+// registers to raw words (emax: the vector's largest exponent field)
 template <class E, int L, class F>
 __device__ __forceinline__ void rf_out(const E (&x)[RfLane<E>::P], int emax,
                                        F store) {
   constexpr int P = RfLane<E>::P;
   if constexpr (RfLane<E>::fixed) {
-    const unsigned nan = emax >= 0x7FF ? 0x7FF80000u : 0u;
     if (emax >= 80 && emax <= 2020) {
 #pragma unroll
       for (int j = 0; j < P; ++j)
-        store(j, fx2d(x[j], emax, rf_log2(L), true, 0u));
+        store(j, fx2d(x[j], emax, rf_log2(L), true));
     } else {
 #pragma unroll
       for (int j = 0; j < P; ++j)
-        store(j, fx2d(x[j], emax, rf_log2(L), false, nan));
+        store(j, fx2d(x[j], emax, rf_log2(L), false));
     }
+  } else if constexpr (Emu<E>::v) {
+#pragma unroll
+    for (int j = 0; j < P; ++j) store(j, df2d_scaled(x[j], emax));
   } else {
 #pragma unroll
     for (int j = 0; j < P; ++j) store(j, x[j]);
@@ -180,7 +206,15 @@ __device__ __forceinline__ void rf_pass(E (&x)[RfLane<E>::P]) {
 #pragma unroll
     for (int u = 0; u < (P >> W); ++u) x[u << W].v += 1ll << (WN - 1);
   }
-  rf_levels<E, P, W>(x);
+  // (double-float: unnormalised inside the pass, one renormalisation at its
+  // end)
+  typedef typename Lazy<E>::type LE;
+  LE v[P];
+#pragma unroll
+  for (int j = 0; j < P; ++j) v[j] = to_lazy(x[j]);
+  rf_levels<LE, P, W>(v);
+#pragma unroll
+  for (int j = 0; j < P; ++j) x[j] = from_lazy(v[j]);
   if constexpr (RfLane<E>::fixed && WN > 0) {
 #pragma unroll
     for (int j = 0; j < P; ++j) x[j].v >>= WN;
@@ -241,6 +275,16 @@ __device__ __forceinline__ void rf_finish(
   constexpr int SL = rf_last<E, L>();
   constexpr int WL = rf_log2(L) - SL;
   typedef typename Sh::Raw Raw;
+  // last pass's points, straight to global memory
+  Raw *dst = (Raw *)p.dst;
+  if (act) {
+    const unsigned m = dA.div((unsigned)gv);
+    const unsigned a = (unsigned)gv - m * (unsigned)p.A;
+    dst += (i64)m * p.ld_dst + (i64)a * p.stride + rf_pos(t, SL, 0, WL);
+  }
+  auto store = [&](int j, Raw y) {
+    if (act) dst[rf_pos(G * (j >> WL), SL, j & ((1 << WL) - 1), WL)] = y;
+  };
   E x[P];
   int emax = 0;
   if constexpr (RfLane<E>::fixed) {
@@ -248,15 +292,33 @@ __device__ __forceinline__ void rf_finish(
     // exponent, restored on store (reduced over the vector's lanes within
     // each warp, then across its warps in shared memory)
     constexpr int WV = G < 32 ? G : 32;
+    int *const smin = sexp + VPC;
     emax = rf_max<P>(d);
+    int emin = emax > 0 ? emax : 0x7FFFFFFF;
+    rf_reduce<WV>(emax, emin);
+    if (threadIdx.x < VPC) {
+      sexp[threadIdx.x] = 0;
+      smin[threadIdx.x] = 0x7FFFFFFF;
+    }
+    __syncthreads();
+    if (t % WV == 0 && emax > 0) {
+      atomicMax(sexp + vl, emax);
+      atomicMin(smin + vl, emin);
+    }
+    __syncthreads();
+    emax = sexp[vl];
+    bool wide = rf_wide(emax, smin[vl]);
+    if constexpr (VPC > 1) wide = __syncthreads_or(wide);
+    emax >>= 20;
+    if (wide) {  // (the whole CTA)
+      df y[P];
+      const int s = emax > 0 ? emax - 1023 : 0;
 #pragma unroll
-    for (int o = WV / 2; o >= 1; o /= 2)
-      emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o, WV));
-    if (threadIdx.x < VPC) sexp[threadIdx.x] = 0;
-    __syncthreads();
-    if (t % WV == 0 && emax > 0) atomicMax(sexp + vl, emax);
-    __syncthreads();
-    emax = sexp[vl] >> 20;
+      for (int r = 0; r < P; ++r) y[r] = d2df_scaled(d[r], s);
+      rf_passes<df, L, 0>(y, reinterpret_cast<df *>(buf), t);
+      rf_out<df, L>(y, s, store);
+      return;
+    }
 #pragma unroll
     for (int r = 0; r < P; ++r) x[r] = d2fx(d[r], emax, rf_w0<E, L>());
   } else {
@@ -264,16 +326,7 @@ __device__ __forceinline__ void rf_finish(
     for (int r = 0; r < P; ++r) x[r] = d[r];
   }
   rf_passes<E, L, 0>(x, buf, t);
-  // last pass's points, straight to global memory
-  if (act) {
-    const unsigned m = dA.div((unsigned)gv);
-    const unsigned a = (unsigned)gv - m * (unsigned)p.A;
-    Raw *dst = (Raw *)p.dst + (i64)m * p.ld_dst + (i64)a * p.stride +
-               rf_pos(t, SL, 0, WL);
-    rf_out<E, L>(x, emax, [&](int j, Raw y) {
-      dst[rf_pos(G * (j >> WL), SL, j & ((1 << WL) - 1), WL)] = y;
-    });
-  }
+  rf_out<E, L>(x, emax, store);
 }
 
 template <class E, int L>
@@ -394,32 +447,56 @@ __device__ __forceinline__ void rs_batch(const RfStep &p, i64 bt, E *xb,
 #pragma unroll
     for (int r = 0; r < P; ++r, q += S) d[r] = *q;
   }
+  Raw *dst = (Raw *)p.dst + (i64)m * p.ld_dst + row0 +
+             (i64)rf_pos(t, SL, 0, WL) * S;
+  auto store = [&](int j, Raw y) {
+    dst[(i64)rf_pos(W * (j >> WL), SL, j & ((1 << WL) - 1), WL) * S] = y;
+  };
+  // (W >= 2: the passes hold at least one exchange, whose barriers also
+  // separate this batch's reads of sexp from the next batch's reset)
+  static_assert(W >= 2, "threads per vector");
   E x[P];
   int emax = 0;
   if constexpr (RfLane<E>::fixed) {
     // fixed point: each vector scaled by the power of two of its largest
     // exponent, restored on store
+    int *const smin = sexp + NV;
     emax = rf_max<P>(d);
-    if (threadIdx.x < NV) sexp[threadIdx.x] = 0;
+    if (threadIdx.x < NV) {
+      sexp[threadIdx.x] = 0;
+      smin[threadIdx.x] = 0x7FFFFFFF;
+    }
     __syncthreads();
-    if (emax > 0) atomicMax(sexp + v, emax);
+    if (emax > 0) {
+      atomicMax(sexp + v, emax);
+      atomicMin(smin + v, emax);
+    }
     __syncthreads();
-    emax = sexp[v] >> 20;
+    emax = sexp[v];
+    bool wide = rf_wide(emax, smin[v]);
+    // (the lanes of a warp see all vectors of the CTA up to 32)
+    if constexpr (NV <= 32)
+      wide = __any_sync(0xffffffffu, wide);
+    else
+      wide = __syncthreads_or(wide);
+    emax >>= 20;
+    if (wide) {  // (the whole CTA)
+      df y[P];
+      const int s = emax > 0 ? emax - 1023 : 0;
+#pragma unroll
+      for (int r = 0; r < P; ++r) y[r] = d2df_scaled(d[r], s);
+      rf_passes<df, L, 0>(y, reinterpret_cast<df *>(buf), t);
+      rf_out<df, L>(y, s, store);
+      return;
+    }
 #pragma unroll
     for (int r = 0; r < P; ++r) x[r] = d2fx(d[r], emax, rf_w0<E, L>());
   } else {
 #pragma unroll
     for (int r = 0; r < P; ++r) x[r] = d[r];
   }
-  // (W >= 2: the passes hold at least one exchange, whose barriers also
-  // separate this batch's reads of sexp from the next batch's reset)
-  static_assert(W >= 2, "threads per vector");
   rf_passes<E, L, 0>(x, buf, t);
-  Raw *dst = (Raw *)p.dst + (i64)m * p.ld_dst + row0 +
-             (i64)rf_pos(t, SL, 0, WL) * S;
-  rf_out<E, L>(x, emax, [&](int j, Raw y) {
-    dst[(i64)rf_pos(W * (j >> WL), SL, j & ((1 << WL) - 1), WL) * S] = y;
-  });
+  rf_out<E, L>(x, emax, store);
 }
 
 template <class E, int L>
@@ -473,7 +550,7 @@ template <class E, int L1, int L2> struct Rf2Mem {
   static constexpr size_t x2 = (size_t)NV2 * RsShape<E, L2>::Lx * sizeof(E);
   static constexpr size_t m01 = slot > x1 ? slot : x1;
   static constexpr size_t region = ((m01 > x2 ? m01 : x2) + 15) / 16 * 16;
-  static constexpr size_t bytes = 16 + region + 4 * (NV2 > 1 ? NV2 : 1);
+  static constexpr size_t bytes = 16 + region + 8 * NV2;
 };
 template <class E, int L1, int L2>
 __host__ __device__ constexpr size_t rf2_smem() {

@@ -945,10 +945,8 @@ __device__ __forceinline__ fx d2fx(double d, int emax, int W) {
   return fx{(((i64)w ^ s) + (i64)(1u + (hi >> 31))) >> 1};
 }
 // fixed point to float64 after K levels, rounded to nearest; plain: no
-// result can leave the float64 range (emax between 80 and 2020), nan: ORed
-// into the high word
-__device__ __forceinline__ double fx2d(fx a, int emax, int K, bool plain,
-                                       unsigned nan) {
+// result can leave the float64 range (emax between 80 and 2020)
+__device__ __forceinline__ double fx2d(fx a, int emax, int K, bool plain) {
   const i64 s = a.v >> 63;
   const unsigned long long u = (unsigned long long)((a.v ^ s) - s);
   const unsigned uh = (unsigned)(u >> 32), ul = (unsigned)u;
@@ -967,7 +965,7 @@ __device__ __forceinline__ double fx2d(fx a, int emax, int K, bool plain,
     }
   }
   if (u == 0) bh = bl = 0u;
-  bh |= ((unsigned)(int)s & 0x80000000u) | nan;
+  bh |= (unsigned)(int)s & 0x80000000u;
   return __hiloint2double((int)bh, (int)bl);
 }
 
