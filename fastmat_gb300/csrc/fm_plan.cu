@@ -1825,10 +1825,13 @@ class Planner {
         st.in_len > L || st.out_len > L)
       return;
     // products in the program index points of a vector, the launch's by
-    // rows: the same when a column holds one vector
+    // rows: the same when a column holds one vector; the kernel conjugates
+    // before the loader's product and after the storer's, so a conjugation in
+    // the program cannot follow or precede a product of the launch
     if ((pre && (st.pre || st.vin.A != 1)) ||
-        (post && (st.post || st.vout.A != 1)) || (cj_in && st.conj_in) ||
-        (cj_out && st.conj_out))
+        (post && (st.post || st.vout.A != 1)) ||
+        (cj_in && (st.conj_in || st.pre)) ||
+        (cj_out && (st.conj_out || st.post)))
       return;
     const int P = fmk::rconv_min_len(ct);
     std::vector<int> rad;
@@ -2048,8 +2051,11 @@ class Planner {
     if (!is_pow2(L) || st.L != L || st.in_len > L || st.out_len > L ||
         st.vin.A * st.vin.Cc != st.V || st.vout.A * st.vout.Cc != st.V)
       return;
-    if ((pre && st.pre) || (post && st.post) || (cj_in && st.conj_in) ||
-        (cj_out && st.conj_out))
+    // (as in try_rconv: conjugation before the loader's product and after the
+    // storer's only)
+    if ((pre && st.pre) || (post && st.post) ||
+        (cj_in && (st.conj_in || st.pre)) ||
+        (cj_out && (st.conj_out || st.post)))
       return;
     const i64 ci = st.vin.Cc, co = st.vout.Cc;
     const i64 wide = 2;  // vectors in a row
