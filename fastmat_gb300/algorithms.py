@@ -48,15 +48,6 @@ class _Iterative:
         arrM = torch.clamp(arrX.abs() - numAlpha, min=0)
         return (arrM / (arrM + numAlpha)) * arrX
 
-    def _residual(self, arrB, arrY):
-        """A y - b (in place on the fresh product where that keeps its
-        type)."""
-        r = self.fmatA.forward(arrY)
-        if (r.dtype == arrB.dtype and r.shape == arrB.shape and
-                not arrB.requires_grad):
-            return r.sub_(arrB)
-        return r - arrB
-
     def _shrink(self, arrY, arrG, numAlpha, arrXold=None, beta=0.0):
         """(step, x, y) of one iteration: step = y - L g, x its soft
         threshold, y = x + beta (x - xold) (None without arrXold).  Column-
@@ -132,7 +123,7 @@ class ISTA(_Iterative):
                                 device=arrB.device).t()
         self.arrB = arrB
         for self.numStep in range(self.numMaxSteps):
-            r = self._residual(arrB, self.arrX)
+            r = A.forward(self.arrX) - arrB
             self.arrStep, self.arrX, _ = self._shrink(
                 self.arrX, A.backward(r), self.numL * self.numLambda * 0.5)
             self.handleCallback(self.cbStep)
@@ -157,7 +148,7 @@ class FISTA(_Iterative):
         self.arrB = arrB
         for self.numStep in range(self.numMaxSteps):
             self.arrXold = self.arrX
-            r = self._residual(arrB, self.arrY)
+            r = A.forward(self.arrY) - arrB
             tOld = self.t
             self.t = (1 + np.sqrt(1 + 4 * self.t ** 2)) / 2
             self.arrStep, self.arrX, self.arrY = self._shrink(
