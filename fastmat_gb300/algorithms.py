@@ -52,10 +52,11 @@ class _Iterative:
         """(step, x, y) of one iteration: step = y - L g, x its soft
         threshold, y = x + beta (x - xold) (None without arrXold).  Column-
         major CUDA tensors of one type take the fused kernel (one launch),
-        anything else separate tensor operations."""
+        anything else, and a softThreshold of the caller's own, separate
+        tensor operations."""
         torch = _torch()
         arrs = [arrY, arrG] + ([] if arrXold is None else [arrXold])
-        if (type(self).softThreshold is _Iterative.softThreshold and
+        if (self.softThreshold is _soft_threshold and
                 isinstance(numAlpha, numbers.Real) and
                 isinstance(self.numL, numbers.Real) and
                 arrY.dtype in (torch.float32, torch.float64,
@@ -108,6 +109,10 @@ class _Iterative:
         if host:
             return np.asfortranarray(res.cpu().numpy())
         return res
+
+
+#: the threshold the fused step computes
+_soft_threshold = _Iterative.softThreshold
 
 
 class ISTA(_Iterative):

@@ -49,3 +49,23 @@ def test_iterates_of_a_user_operator():
         y = x + (s - 1) / t * (x - old)
     want = torch.where(x != 0, z, x)
     assert float((got - want).abs().max()) <= 1e-14
+
+
+@pytest.mark.gpu
+def test_a_threshold_set_as_a_parameter_is_used():
+    import fastmat_gb300 as fm
+    from fastmat_gb300.algorithms import ISTA
+
+    def halve(x, alpha):
+        halve.calls += 1
+        return 0.5 * x
+
+    halve.calls = 0
+    rng = np.random.default_rng(0)
+    op = fm.Circulant(rng.standard_normal(64))
+    b = torch.from_numpy(rng.standard_normal((3, 64))).to(
+        torch.complex128).cuda().t()
+    alg = ISTA(op, numMaxSteps=3, softThreshold=halve)
+    alg.process(b)
+    assert halve.calls == 3
+    assert torch.equal(alg.arrX, 0.5 * alg.arrStep)
