@@ -197,6 +197,8 @@ class Matrix:
     """
 
     _array = None
+    #: tensor dtype -> _io_types() (absent in pickles of earlier versions)
+    _io = None
 
     def __init__(self, arrMatrix, **options):
         if not isinstance(arrMatrix, np.ndarray):
@@ -219,7 +221,7 @@ class Matrix:
                 "precision must be 'native', 'fp64', 'fp32' or 'bf16'")
         self._precision = prec
         self._plans = {}
-        self._io = {}   # tensor dtype -> _io_types()
+        self._io = None
 
     def _getProperties(self):
         return {'minType': self._minType, 'precision': self._precision}
@@ -343,6 +345,8 @@ class Matrix:
         the plan's compute code).  It depends on the operator's type and
         options alone, which do not change, so it is worked out once per
         tensor dtype."""
+        if self._io is None:
+            self._io = {}
         io = self._io.get(tdt)
         if io is None:
             in_dt = _numpy_dtype(tdt)
