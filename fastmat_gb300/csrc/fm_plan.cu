@@ -20,6 +20,7 @@
 #include <cstdio>
 #include <cstring>
 #include <atomic>
+#include <iterator>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -1957,11 +1958,15 @@ class Planner {
     return rx_w_[key] = p;
   }
   // spectra in the order the lanes hold the forward transform's results
-  const void *rx_spectrum(const void *in, int L, i64 n, i64 stride) {
-    const int P = fmk::kRxP, G = L / P;
+  std::vector<int> rx_radices(int L) {
     std::vector<int> rad;
     for (int rest = L; rest > 1; rest /= rad.back())
-      rad.push_back(std::min(rest, P));
+      rad.push_back(std::min(rest, fmk::kRxP));
+    return rad;
+  }
+  const void *rx_spectrum(const void *in, int L, i64 n, i64 stride) {
+    const int P = fmk::kRxP, G = L / P;
+    const std::vector<int> rad = rx_radices(L);
     const Perm &pm = perm_for(rad);
     const int R = rad.back();  // last stage: M = 1
     std::vector<int> perm((size_t)L);
@@ -2067,8 +2072,39 @@ class Planner {
           L > (ci == 1 ? fmk::rxfft_max_turn : fmk::rxfft_max))
         return;
     }
+    // the tables (one four-step table per (N, N2), entry j N2 + q of row
+    // j < N1: the pass over vectors of N1 points has j the point and q the
+    // vector, the pass over vectors of N2 points the reverse)
+    const bool per = sm && sm->mod != 1;
+    const void *stw = nullptr, *spec = nullptr, *w = nullptr;
+    if (sm) perm_for(rx_radices(L));  // (shared with the vector program)
+    const size_t before = P_->allocs.size();
+    const i64 bytes = P_->const_bytes;
+    try {
+      stw = rx_twiddle(L);
+      if (sm)
+        spec = rx_spectrum(sm->ptr, L, per ? st.V : 1, sm->stride);
+      if (tw) w = rx_wtab(tw->N, ci != 1 ? st.V : (i64)L);
+    } catch (const Error &e) {
+      // no room for tables that the vector program does without (up to 32
+      // bytes a point): it runs the launch, and the room is given back
+      if (e.code != FM_ERR_NOMEM) throw;
+      cudaGetLastError();
+      CUDA_TRY(cudaDeviceSynchronize());  // the tables' kernels
+      for (size_t k = before; k < P_->allocs.size(); ++k) {
+        const void *p = P_->allocs[k];
+        for (auto t = rx_tw_.begin(); t != rx_tw_.end();)
+          t = t->second == p ? rx_tw_.erase(t) : std::next(t);
+        for (auto t = rx_w_.begin(); t != rx_w_.end();)
+          t = t->second == p ? rx_w_.erase(t) : std::next(t);
+        cudaFree(P_->allocs[k]);
+      }
+      P_->allocs.resize(before);
+      P_->const_bytes = bytes;
+      return;
+    }
     ls.rc_L = L;
-    ls.rc_tw = rx_twiddle(L);
+    ls.rc_tw = stw;
     ls.rc_pre = pre;
     ls.rc_post = post;
     ls.rx_pre_pt = pre != nullptr;
@@ -2077,24 +2113,14 @@ class Planner {
     ls.rc_conj_out = cj_out;
     ls.rc_sign = sign;
     if (sm) {
-      const bool per = sm->mod != 1;
-      ls.rc_spec = rx_spectrum(sm->ptr, L, per ? st.V : 1, sm->stride);
+      ls.rc_spec = spec;
       ls.rx_spec_stride = per ? L : 0;
       ls.rc_spec_conj = sm->sign;
     }
     if (tw) {
-      // one table per (N, N2), entry j N2 + q of row j < N1: the pass over
-      // vectors of N1 points has j the point and q the vector, the pass over
-      // vectors of N2 points the reverse
-      if (ci != 1) {
-        ls.rx_w = rx_wtab(tw->N, st.V);
-        ls.rx_wq = 1;
-        ls.rx_wj = st.V;
-      } else {
-        ls.rx_w = rx_wtab(tw->N, L);
-        ls.rx_wq = L;
-        ls.rx_wj = 1;
-      }
+      ls.rx_w = w;
+      ls.rx_wq = ci != 1 ? 1 : L;
+      ls.rx_wj = ci != 1 ? st.V : 1;
       ls.rx_w_sign = tw->sign;
     }
     ls.kind = sm ? 6 : 5;
