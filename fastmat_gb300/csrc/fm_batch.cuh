@@ -29,6 +29,17 @@ enum {
   RXM_FFT = 1,    // as rxfft_kernel, 64..512 points
   RXM_CONV = 2    // as rxconv_kernel, 128..4096 points
 };
+// The lengths built, for the dispatch on the device and for the rule that
+// sends a step there: a step never meets a length that is not built.
+#define FM_RXB_FFT(X) X(64) X(128) X(256) X(512)
+#define FM_RXB_CONV(X) X(128) X(256) X(512) X(1024) X(2048) X(4096)
+inline bool rxb_built(int mode, int L) {
+#define FM_RXB_IS(N) || L == N
+  return mode == RXM_FFT    ? false FM_RXB_FFT(FM_RXB_IS)
+         : mode == RXM_CONV ? false FM_RXB_CONV(FM_RXB_IS)
+                            : false;
+#undef FM_RXB_IS
+}
 constexpr int kRxbPoints = FM_MAX_THREADS * kRxP;  // points per tile
 // shared memory of a tile's exchange buffers
 constexpr size_t kRxbBytes = 38400;
@@ -224,16 +235,14 @@ __device__ __forceinline__ void rxb_conv(const RxStep &p, cfp<8> *xb,
 __device__ __forceinline__ void rx_batch_tile(const RxStep &p, int mode,
                                            cfp<8> *xb, unsigned tile) {
   switch (mode * 8192 + p.L) {
-    case RXM_FFT * 8192 + 64: rxb_fft<64>(p, xb, tile); break;
-    case RXM_FFT * 8192 + 128: rxb_fft<128>(p, xb, tile); break;
-    case RXM_FFT * 8192 + 256: rxb_fft<256>(p, xb, tile); break;
-    case RXM_FFT * 8192 + 512: rxb_fft<512>(p, xb, tile); break;
-    case RXM_CONV * 8192 + 128: rxb_conv<128>(p, xb, tile); break;
-    case RXM_CONV * 8192 + 256: rxb_conv<256>(p, xb, tile); break;
-    case RXM_CONV * 8192 + 512: rxb_conv<512>(p, xb, tile); break;
-    case RXM_CONV * 8192 + 1024: rxb_conv<1024>(p, xb, tile); break;
-    case RXM_CONV * 8192 + 2048: rxb_conv<2048>(p, xb, tile); break;
-    case RXM_CONV * 8192 + 4096: rxb_conv<4096>(p, xb, tile); break;
+#define FM_RXB_CASE(N) \
+  case RXM_FFT * 8192 + N: rxb_fft<N>(p, xb, tile); break;
+    FM_RXB_FFT(FM_RXB_CASE)
+#undef FM_RXB_CASE
+#define FM_RXB_CASE(N) \
+  case RXM_CONV * 8192 + N: rxb_conv<N>(p, xb, tile); break;
+    FM_RXB_CONV(FM_RXB_CASE)
+#undef FM_RXB_CASE
     default: break;
   }
 }

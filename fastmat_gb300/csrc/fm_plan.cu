@@ -3777,10 +3777,12 @@ int fm_batch_create(int32_t num_ops, fm_plan *const *plans,
         fmk::RxStep rx;
         memset(&rx, 0, sizeof(rx));
         if (ctype == FM_C64 && st.src_type == FM_C64 &&
-            st.dst_type == FM_C64 && !st.accumulate && !st.has_scale &&
-            ((ls0.kind == 5 && ls0.rc_L >= 64 && ls0.rc_L <= 512) ||
-             (ls0.kind == 6 && ls0.rc_L >= 128))) {
-          rxmode = ls0.kind == 5 ? fmk::RXM_FFT : fmk::RXM_CONV;
+            st.dst_type == FM_C64 && !st.accumulate && !st.has_scale)
+          rxmode = ls0.kind == 5   ? fmk::RXM_FFT
+                   : ls0.kind == 6 ? fmk::RXM_CONV
+                                   : fmk::RXM_NONE;
+        if (!fmk::rxb_built(rxmode, ls0.rc_L)) rxmode = fmk::RXM_NONE;
+        if (rxmode) {
           rx = rx_step(ls0, st);
           // an FFT tile is one or two groups of adjacent vectors of a
           // column, a convolution tile any consecutive vectors
