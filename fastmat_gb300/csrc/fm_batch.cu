@@ -1,7 +1,8 @@
 // Launcher of the batched persistent kernel (many operators in one
 // cooperative launch; see batch_kernel in fm_batch.cuh).  The instantiations
 // live in translation units of their own (fm_batch_c64_pow2.cu,
-// fm_batch_c64.cu, fm_batch_c64_gen.cu, fm_batch_df.cu), which compile in parallel.
+// fm_batch_c64.cu, fm_batch_c64_gen.cu, fm_batch_df.cu), which compile in
+// parallel.
 
 #include <cuda_runtime.h>
 

@@ -39,7 +39,8 @@ cudaError_t launch_batch_one(const BatchLaunch &b, cudaStream_t s) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, fn, b.steps, b.start, b.level, b.rx,
-                            b.rxmode, b.nlev, b.bar, b.err, b.max_B, b.max_tile, b.wait_limit);
+                            b.rxmode, b.nlev, b.bar, b.err, b.max_B,
+                            b.max_tile, b.wait_limit);
 }
 
 }  // namespace fmk

@@ -1998,7 +1998,7 @@ class Planner {
   // a power of two they are built for.  Lines of the rule: rows of two or
   // more adjacent vectors (a Fourier mode of 256 points, 2^20 x 8: at 2
   // vectors a row 88 us on the stage kernel's tiles, 49 here in complex64, 214
-  // and 109 in double-float; at 8 vectors 76 and 32, 200 and 101; whole
+  // and 112 in double-float; at 8 vectors 76 and 32, 200 and 104; whole
   // convolutions of 4096 points, 256 columns in double-float, 112 and 40).
   // A plain Fourier mode of a Kron above 512 points, and a whole Fourier
   // column in one launch, stay on the stage kernel's tiles, whose copies the
@@ -2661,7 +2661,6 @@ void launch_step(fm_plan *P, LStep &ls, fmk::Step &st, cudaStream_t s) {
         pr.ctr = P->pair_ctr;
         pr.err = P->err;
         pr.wait_limit = P->wait_limit;
-        pr.lag = 1;  // set by the launcher from the resident grid
         CUDA_TRY(cudaMemsetAsync(P->pair_ctr, 0,
                                  (size_t)(1 + st.num_cols) * 4, s));
         CUDA_TRY(fmk::launch_rfwht2(ls.rc_ct, pr, s));
@@ -2767,7 +2766,6 @@ void launch_step(fm_plan *P, LStep &ls, fmk::Step &st, cudaStream_t s) {
       pr.blocks = blocks;
       pr.n1 = ls.rc2_n1;
       pr.n2 = ls.rc2_n2;
-      pr.lag = 1;  // set by the launcher from the resident grid
       CUDA_TRY(cudaMemsetAsync(P->pair_ctr, 0, (size_t)(1 + blocks) * 4, s));
       CUDA_TRY(fmk::launch_rkch(P->ctype, pr, s));
       P->pair_done = true;

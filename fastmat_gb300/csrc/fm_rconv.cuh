@@ -282,10 +282,12 @@ __device__ __forceinline__ void rc_inverse(E (&x)[RcLane<E>::P], E *buf, int g,
 // The double-float kernels are bound by instruction issue and the integer
 // pipe (Kron(F256, H8, C128), 8 columns, before: 0.62 issued per cycle, ALU
 // 48 %, FMA 37 %): packed arithmetic (one instruction for both parts) and
-// the conversions below (13 + 19 instead of about 15 + 31 instructions per
+// the conversions below (14 + 21 instead of about 15 + 31 instructions per
 // real word, no FP64 addition) took its step from 3.70 to 2.61 ms, this
-// kernel's launch from 1850 to 1015 us; the FMA pipe is now 74 % busy (about
-// 410 FP32 operations per element, 720 us at its full rate).  (A barrier per
+// kernel's launch from 1850 to 1015 us; 1062 us with products normalised as
+// the scalar ones, Inf and NaN kept and the flush of heads and tails apart
+// (about 420 FP32 operations per element, 740 us at the FMA pipe's full
+// rate).  (A barrier per
 // batch to keep the warps of a CTA on the same instructions measured 2.62 ms
 // for the step and is left out.)
 // ---- raw points of a double-float vector (complex128 words) and the

@@ -31,14 +31,15 @@
 // Measured against the stage kernel's tiles (vprog_kernel, every radix stage
 // a pass over shared memory with run-time index arithmetic), microseconds
 // per launch: 32 columns of 2^18 points, double-float, strided 512 points
-// 347 -> 134 (with gathers and products around), convolution of 512 points
-// 558 -> 185; the same in complex64 118 -> 35 and 62 -> 43; convolution of
-// 4096 points, 4 columns, double-float 57 -> 19.  Eight points a thread in
+// 347 -> 132 (with gathers and products around), convolution of 512 points
+// 558 -> 207 (185 before products were normalised and heads rounded); the
+// same in complex64 118 -> 35 and 62 -> 43; convolution of 4096 points, 4
+// columns, double-float 57 -> 22.  Eight points a thread in
 // complex64 too: 16 (the radices 16, 16, 2) measured 6 % further from 64-bit
 // results over 2^18 points, and spilled in the convolution.  The next batch
 // is copied ahead (strided complex64 38 -> 35, gathered double-float 168 ->
-// 134).  Bounds: the FMA pipe in double-float (67 % busy in the convolution,
-// 47 % in the FFT passes, whose table loads and barriers 16 warps a
+// 134).  Bounds: the FMA pipe in double-float (66 % busy in the convolution,
+// 46 to 50 % in the FFT passes, whose table loads and barriers 16 warps a
 // multiprocessor do not cover), the shared-memory / L1 pipe in complex64 (50
 // to 69 %).  Measured and left out, in double-float: intermediates as packed
 // double-floats instead of float64 words (no change: the conversions run in
@@ -139,8 +140,7 @@ __device__ __forceinline__ float2 rx_zero(float2) {
 
 // P points j0 + dj r of one vector of the input view (row of point 0: rb,
 // column offset col) from any type, zero outside the vector or the column
-// (RAW: the buffer is known to hold the kernel's own type)
-template <class E, int L, bool RAW = false>
+template <class E, int L>
 __device__ __forceinline__ void rx_load(
     typename RxRaw<E>::type (&d)[RcLane<E>::P], const RxStep &p, bool act,
     i64 col, i64 rb, int j0, int dj) {
@@ -154,12 +154,7 @@ __device__ __forceinline__ void rx_load(
     Raw v = rx_zero(Raw());
     if (act && j < p.in_len && row < p.in_rows) {
       const i64 srow = p.map_in ? p.map_in[row] : row;
-      if (srow >= 0) {
-        if constexpr (RAW)
-          v = ((const Raw *)p.src)[col + srow];
-        else
-          v = load_as<Raw>(p.src, p.src_type, col + srow);
-      }
+      if (srow >= 0) v = load_as<Raw>(p.src, p.src_type, col + srow);
     }
     d[r] = v;
   }

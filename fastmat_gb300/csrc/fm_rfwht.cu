@@ -1,7 +1,7 @@
 // Instantiations and launchers of the register-resident FWHT kernels
-// (fm_rfwht.cuh): float32 and fixed-point (float64) real data, contiguous vectors of
-// 1024..8192 (float32) or 256..8192 (fixed-point (float64)) points, strided vectors
-// of 64..2048 (float32) or 32..1024 (fixed-point (float64)) points.
+// (fm_rfwht.cuh): float32 and float64 (fixed-point) real data, contiguous
+// vectors of 1024..8192 (float32) or 256..8192 (float64) points, strided
+// vectors of 64..2048 (float32) or 32..1024 (float64) points.
 #include <map>
 #include <mutex>
 #include <tuple>

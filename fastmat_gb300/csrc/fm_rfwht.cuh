@@ -4,10 +4,12 @@
 // data (64-bit fixed point, see fx in fm_types.cuh: float64 launches were
 // bound by the double-float additions and conversions; Hadamard(18) on 48
 // columns 224 -> 129 us, the FWHT mode of Kron(F256, H8, C128) on 8 complex
-// columns 875 -> 532 us, errors against 64 bits 7.2e-15 -> 1.3e-15; 99.5 and
-// 451 us with the later changes below).  The float64 kernels are bound by the
-// integer pipe (66 % busy in the strided one), the float32 ones by barriers
-// and the shared-memory pipe (55-60 % busy).
+// columns 875 -> 532 us, errors against 64 bits 7.2e-15 -> 2.3e-16; 105 and
+// 494 us with the later changes below, 99.5 and 451 before the points were
+// rounded between passes and vectors of wide range told apart, rf_wide).  The
+// float64 kernels are bound by the integer pipe (71 % busy in the strided
+// one), the float32 ones by barriers and the shared-memory pipe (55-60 %
+// busy).
 //
 //   * a vector of L points is held by G = L / P threads of a CTA, P points
 //     per thread (32 float or 16 fixed-point); the CTA works on
@@ -116,8 +118,9 @@ __device__ __forceinline__ int rf_max(const double (&d)[P]) {
 // 2^-60 of the largest, 48 bits of those down to 2^-11; where whole groups are
 // smaller, the large elements may cancel in some results, which then hang on
 // the small ones' own bits.  Random data never gets here (a group of 16
-// normal variates: 2^-150); the double-float form of Hadamard(18) x 48 takes
-// about twice the time.
+// normal variates: 2^-150); Hadamard(18) x 48 with one large element every
+// 4096 rows takes 142 us where normal data takes 106 (231 with every pass in
+// double-float).
 __device__ __forceinline__ bool rf_wide(int mx, int mn) {
   return mx >= 0x7FF00000 || (mn >> 20) + 11 < (mx >> 20);
 }
@@ -521,7 +524,7 @@ __global__ void __launch_bounds__(RsShape<E, L>::T, (RsOcc<E, L>::v))
 // by the second) is still in L2 when the second pass reads it.  Work items
 // are handed out in order by an atomic counter: the first-pass items of
 // column k (one vector each), then the second-pass items of column k - lag
-// (NV2 strided vectors each; the launcher sets the lag).  A second-pass item of column m waits until
+// (NV2 strided vectors each).  A second-pass item of column m waits until
 // all first-pass items of column m have finished (their count in ctr[1 +
 // m], raised with release semantics after each item's stores; read with
 // acquire semantics, polls bounded by wait_limit).  Every awaited item was
@@ -533,7 +536,8 @@ struct RfPair {
   unsigned *ctr;   // [0] items handed out, [1 + m] first-pass items done
   int *err;
   long long wait_limit;
-  int lag;         // columns between a column's first and second pass
+  int lag = 0;     // columns between a column's first and second pass (set
+                   // by the launcher from the resident grid)
 };
 #define FM_RF2_THREADS 256
 

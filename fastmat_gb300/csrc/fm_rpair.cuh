@@ -31,7 +31,7 @@ struct RchPair {
   long long wait_limit;
   i64 blocks;      // blocks over all columns
   int n1, n2;      // convolution / FWHT items per block
-  int lag;         // blocks between a block's first and second mode
+  int lag = 0;         // blocks between a block's first and second mode
 };
 
 #define FM_RCH_THREADS 256

@@ -53,7 +53,8 @@ template <class E> struct RsfOcc {
 };
 // double-float copies the next batch ahead into shared memory while the
 // current one transforms (its two CTAs per SM leave the load latency
-// uncovered: FFT(256) at stride 32768 on 8 columns 710 -> 615 us); complex64,
+// uncovered: FFT(256) at stride 32768 on 8 columns 710 -> 615 us, 628 with
+// the wider conversions); complex64,
 // at 0.93 of the copy peak, loads straight into registers
 template <class E> struct RsfAhead { static constexpr bool v = Emu<E>::v; };
 template <class E, int L>

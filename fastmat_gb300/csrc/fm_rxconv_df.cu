@@ -1,4 +1,5 @@
-// Instantiations and launcher of rxconv_kernel (fm_rfft.cuh): packed double-float.
+// Instantiations and launcher of rxconv_kernel (fm_rfft.cuh): packed
+// double-float.
 #include "fm_launch.cuh"
 #include "fm_rfft.cuh"
 

@@ -373,7 +373,7 @@ struct FDiv : FDivB {
 // Divisors built per stage or per tile: the quotient of m is estimated in
 // float (within 2^10) and corrected by its remainder, since a 64-bit division
 // in every thread takes the FP64 pipe, the slowest of this GPU (Fourier(6000)
-// x 64: 15 % of its cycles busy there; 30.8 -> 28.7 us without).
+// x 64: 15 % of its cycles busy there; 30.7 us with it, 30.0 without).
 struct FDivF : FDivB {
   __device__ __forceinline__ explicit FDivF(unsigned d_) {
     d = d_;
@@ -514,15 +514,15 @@ __device__ __forceinline__ LC cmul_lazy(LC a, C w) {
       return rmul(a, b.h.x, b.l.x) +
              rmul(rot90(a, SG < 0 ? +1 : -1), b.h.y, b.l.y);
     } else {
-    LC r;
-    if constexpr (SG < 0) {
-      r.x = a.x * b.x - a.y * b.y;
-      r.y = a.x * b.y + a.y * b.x;
-    } else {
-      r.x = a.x * b.x + a.y * b.y;
-      r.y = a.y * b.x - a.x * b.y;
-    }
-    return r;
+      LC r;
+      if constexpr (SG < 0) {
+        r.x = a.x * b.x - a.y * b.y;
+        r.y = a.x * b.y + a.y * b.x;
+      } else {
+        r.x = a.x * b.x + a.y * b.y;
+        r.y = a.y * b.x - a.x * b.y;
+      }
+      return r;
     }
   }
 }
